@@ -326,3 +326,72 @@ def tolerance(case):
     if case["kind"] in ("input", "order", "rowwise") or case["pooling"] == "none":
         return "exact"
     return {"fp32": {"rel": 2.5e-5}, "fp16": {"rel": 8e-4}, "bf16": {"rel": 7e-3}}[case["output"]]
+
+
+# ---- the same in 64 bits ----------------------------------------------------------------------------------
+
+def _decoded(rows, ty, dim):
+    """Table rows (bytes) as float64 [n, dim]."""
+    n = rows.shape[0]
+    if ty in ("fp32", "fp16"):
+        dtype, size = (torch.float32, 4) if ty == "fp32" else (torch.float16, 2)
+        return rows[:, :size * dim].contiguous().view(dtype).view(n, dim).double()
+    if ty == "fp8":
+        b = torch.arange(256, device=rows.device)
+        e, m, sign = (b >> 3) & 15, (b & 7).double(), 1.0 - 2.0 * (b >> 7).double()
+        values = sign * torch.where(e > 0, (1.0 + m / 8.0) * torch.exp2((e - 7).double()), m / 8.0 * 2.0 ** -6)
+        return values[rows[:, :dim].long()]
+    header = rows[:, :4].contiguous().view(torch.float16).view(n, 2).double()
+    bits = {"int8": 8, "int4": 4, "int2": 2}[ty]
+    shifts = torch.arange(0, 8, bits, device=rows.device, dtype=torch.uint8)
+    codes = ((rows[:, 4:4 + (dim * bits + 7) // 8].unsqueeze(-1) >> shifts) & (2 ** bits - 1)).flatten(1)[:, :dim]
+    return codes.double() * header[:, :1] + header[:, 1:]
+
+
+def _exact_lookup(case, s, indices, offsets):
+    ws, types = _spec(case, 0), case["types"].split(",")
+    pooled, column = case["pooling"] != "none", 0
+    bounds = offsets[:: ws.B].tolist()
+    out = torch.zeros(ws.B if pooled else indices.numel(), sum(ws.dims) if pooled else max(ws.dims), dtype=torch.float64, device=indices.device)
+    for t, dim in enumerate(ws.dims):
+        rows, mine = s["tables"].table_rows(t), offsets[t * ws.B:(t + 1) * ws.B + 1].long()
+        for lo in range(bounds[t], bounds[t + 1], 1 << 20):
+            hi = min(bounds[t + 1], lo + (1 << 20))
+            i = indices[lo:hi].long()
+            x = _decoded(rows[i.clamp(min=0)], types[t % len(types)], dim) * (i >= 0).unsqueeze(1)
+            if not pooled:
+                out[lo:hi, :dim] = x
+                continue
+            if s["weights"] is not None:
+                x *= s["weights"][lo:hi].unsqueeze(1)
+            bag = torch.searchsorted(mine, torch.arange(lo, hi, device=i.device), right=True) - 1
+            out[:, column:column + dim].index_add_(0, bag, x)
+        if case["pooling"] == "mean":
+            out[:, column:column + dim] /= (mine[1:] - mine[:-1]).clamp(min=1).unsqueeze(1)
+        column += dim
+    return out
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, from the tables' bytes in float64; None where the outputs are bytes, indices
+    or copies."""
+    kind = case["kind"]
+    if kind not in ("lookup", "request") and not (kind == "rowwise" and case["op"].startswith("dequantize")):
+        return None
+    s = prepare(case, seed)
+    if kind == "lookup":
+        return _exact_lookup(case, s, s["indices"], s["offsets"])
+    if kind == "rowwise":
+        x = s["x"]
+        if case["op"] == "dequantize8":
+            header = x[:, -8:].contiguous().view(torch.float32).double()
+            return x[:, :-8].double() * header[:, :1] + header[:, 1:]
+        return _decoded(torch.cat([x[:, -4:], x[:, :-4]], 1), "int4", case["cols"])
+    order = s["permute"].tolist()
+    parts = torch.split(s["values"], s["lengths"].sum(1).tolist())
+    lengths = s["lengths"][s["permute"].long()].view(-1)
+    offsets = torch.zeros(lengths.numel() + 1, dtype=torch.int64, device=lengths.device)
+    offsets[1:] = torch.cumsum(lengths, 0)
+    pooled = _exact_lookup(case, s, torch.cat([parts[t] for t in order]), offsets)
+    pieces = torch.split(pooled, _spec(case, 0).dims, 1)
+    return torch.cat([pieces[f] for f in s["order"]._permute.tolist()], 1)
