@@ -410,29 +410,44 @@ __global__ void __launch_bounds__(kBigThreads, kBigBlocksPerSM) big_tile_scan_ke
 
 // ---- permute 2D sparse data ----------------------------------------------------------------------------
 
-// seg_len[t] += sum of a slice of lengths[t, :]  (seg_len cleared beforehand)
+// What stands in front of the copy, in two launches: the tables' partial sums, then one block that turns them into the
+// tables' offsets while the other blocks copy the rows of `lengths` (they need no offsets).  Small
+// requests take one launch of one block that does both, and nothing has to be cleared in either form (the
+// sums of a table are added up from its partial sums, not with atomics).
+
+constexpr int kMaxPartials = 32;             // blocks that add up one table's lengths
+constexpr int kOffsetThreads = 256;
+constexpr int kSmallThreads = 1024;
+// The one-block form takes up to this many tables, lengths per table and lengths in all: a warp then reads at most 16
+// lines of a table, and four tables one after the other, which is what the launches it saves cost.
+constexpr int64_t kSmallTables = 128, kSmallBatch = 512, kSmallLengths = 16384;
+inline bool small_request(int64_t T_in, int64_t T_out, int64_t B)
+{
+    return T_in <= kSmallTables && T_out <= kSmallTables && B <= kSmallBatch && T_in * B <= kSmallLengths && T_out * B <= kSmallLengths;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) segment_lengths_kernel(const T* __restrict__ lengths, int64_t B, int64_t* __restrict__ seg_len)
+__global__ void __launch_bounds__(256) segment_partials_kernel(const T* __restrict__ lengths, int64_t B, int64_t* __restrict__ partials)
 {
     __shared__ int64_t red[8];
     const int64_t t = blockIdx.y;
     const T* row = lengths + t * B;
     int64_t s = 0;
-    for (int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b < B; b += static_cast<int64_t>(gridDim.x) * blockDim.x)
+#pragma unroll 8
+    for (int64_t b = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; b < B; b += static_cast<int64_t>(gridDim.x) * 256)
         s += static_cast<int64_t>(row[b]);
     s = block_sum(s, red);
-    if (threadIdx.x == 0 && s != 0) atomicAdd(reinterpret_cast<unsigned long long*>(seg_len + t), static_cast<unsigned long long>(s));
+    if (threadIdx.x == 0) partials[t * gridDim.x + blockIdx.x] = s;
 }
 
-// One block: in_off = exclusive sums of seg_len over the input tables; out_off = exclusive sums of
-// seg_len[permute[i]] over the output tables.  An entry of `permute` outside [0, T_in) counts as an empty table
-// and sets the error flag.
-__global__ void __launch_bounds__(kScanThreads) segment_offsets_kernel(const int64_t* __restrict__ seg_len, int64_t T_in,
-                                                                        const int32_t* __restrict__ permute, int64_t T_out,
-                                                                        int64_t* __restrict__ in_off, int64_t* __restrict__ out_off,
-                                                                        int32_t* error_flag)
+// One block of THREADS threads: in_off = exclusive sums of the tables' lengths over the input tables; out_off = exclusive
+// sums of the lengths of tables permute[i] over the output tables.  An entry of `permute` outside [0, T_in) counts as an
+// empty table and sets the error flag.  `length_of(t)` gives the length of input table t.
+template <int THREADS, typename LengthOf>
+__device__ __forceinline__ void segment_offsets(LengthOf length_of, int64_t T_in, const int32_t* __restrict__ permute, int64_t T_out,
+                                                int64_t* in_off, int64_t* out_off, int32_t* error_flag)
 {
-    __shared__ int64_t warp_base[kScanThreads / 32];
+    __shared__ int64_t warp_base[THREADS / 32];
     __shared__ int64_t carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int pass = 0; pass < 2; ++pass) {
@@ -443,15 +458,15 @@ __global__ void __launch_bounds__(kScanThreads) segment_offsets_kernel(const int
             off[0] = 0;
         }
         __syncthreads();
-        for (int64_t base = 0; base < count; base += kScanThreads) {
+        for (int64_t base = 0; base < count; base += THREADS) {
             const int64_t i = base + threadIdx.x;
             int64_t v = 0;
             if (i < count) {
                 if (pass == 0) {
-                    v = seg_len[i];
+                    v = length_of(i);
                 } else {
                     const int64_t p = permute[i];
-                    if (p >= 0 && p < T_in) v = seg_len[p];
+                    if (p >= 0 && p < T_in) v = in_off[p + 1] - in_off[p];     // written by this block in the first pass
                     else if (error_flag) atomicOr(error_flag, 1);
                 }
             }
@@ -467,26 +482,73 @@ __global__ void __launch_bounds__(kScanThreads) segment_offsets_kernel(const int
             for (int w = 0; w < warp; ++w) run += warp_base[w];
             if (i < count) off[i + 1] = run;
             __syncthreads();
-            if (threadIdx.x == kScanThreads - 1) carry = run;
+            if (threadIdx.x == THREADS - 1) carry = run;
             __syncthreads();
         }
     }
 }
 
+// Block (0, 0) makes the offsets; block (1 + x, y) copies slice x of row y of the permuted `lengths`.
 template <typename T>
-__global__ void __launch_bounds__(256) permute_lengths_kernel(const T* __restrict__ lengths, int64_t T_in, int64_t B,
-                                                              const int32_t* __restrict__ permute, T* __restrict__ out)
+__global__ void __launch_bounds__(kOffsetThreads) offsets_and_lengths_kernel(const int64_t* __restrict__ partials, int per_table,
+                                                                             const T* __restrict__ lengths, int64_t T_in, int64_t B,
+                                                                             const int32_t* __restrict__ permute, int64_t T_out,
+                                                                             T* __restrict__ out, int64_t* in_off, int64_t* out_off,
+                                                                             int32_t* error_flag)
 {
+    if (blockIdx.x == 0) {
+        if (blockIdx.y != 0) return;
+        segment_offsets<kOffsetThreads>(
+            [&](int64_t t) {
+                int64_t v = 0;
+                for (int g = 0; g < per_table; ++g) v += partials[t * per_table + g];
+                return v;
+            },
+            T_in, permute, T_out, in_off, out_off, error_flag);
+        return;
+    }
     const int64_t i = blockIdx.y;
     const int64_t p = permute[i];
     const bool ok = p >= 0 && p < T_in;
-    for (int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b < B; b += static_cast<int64_t>(gridDim.x) * blockDim.x)
+#pragma unroll 4
+    for (int64_t b = static_cast<int64_t>(blockIdx.x - 1) * kOffsetThreads + threadIdx.x; b < B;
+         b += static_cast<int64_t>(gridDim.x - 1) * kOffsetThreads)
         out[i * B + b] = ok ? lengths[p * B + b] : static_cast<T>(0);
+}
+
+// The same by one block: a warp adds up a table at a time, then the offsets, then the rows.
+template <typename T>
+__global__ void __launch_bounds__(kSmallThreads) small_offsets_and_lengths_kernel(const T* __restrict__ lengths, int64_t T_in, int64_t B,
+                                                                                  const int32_t* __restrict__ permute, int64_t T_out,
+                                                                                  T* __restrict__ out, int64_t* in_off, int64_t* out_off,
+                                                                                  int32_t* error_flag)
+{
+    __shared__ int64_t table_len[kSmallTables];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t t = warp; t < T_in; t += kSmallThreads / 32) {
+        int64_t s = 0;
+#pragma unroll 8
+        for (int64_t b = lane; b < B; b += 32) s += static_cast<int64_t>(lengths[t * B + b]);
+        s = warp_sum(s);
+        if (lane == 0) table_len[t] = s;
+    }
+    __syncthreads();
+    segment_offsets<kSmallThreads>([&](int64_t t) { return table_len[t]; }, T_in, permute, T_out, in_off, out_off, error_flag);
+    for (int64_t i = warp; i < T_out; i += kSmallThreads / 32) {
+        const int64_t p = permute[i];
+        const bool ok = p >= 0 && p < T_in;
+#pragma unroll 8
+        for (int64_t b = lane; b < B; b += 32) out[i * B + b] = ok ? lengths[p * B + b] : static_cast<T>(0);
+    }
 }
 
 // Output position o lies in output table i with out_off[i] <= o < out_off[i + 1]; its source is
 // in_off[permute[i]] + (o - out_off[i]).  A thread finds the table of its first position by binary search
 // and walks forward from there.  VT is the unit copied per position (the element, or 16 bytes of a wide row).
+//
+// A chunk that lies inside one table -- nearly all of them -- is copied with all of a thread's loads (64 bytes) in front of
+// its first store and no per-element test; the chunks that hold a boundary are walked element by element.
+constexpr int kSegmentBytesPerThread = 64;
 template <typename VT, bool ONE_UNIT>
 __global__ void __launch_bounds__(256) permute_segments_kernel(const VT* __restrict__ src, VT* __restrict__ dst, int64_t units_per_pos,
                                                                int64_t capacity /* positions */, const int32_t* __restrict__ permute,
@@ -494,30 +556,43 @@ __global__ void __launch_bounds__(256) permute_segments_kernel(const VT* __restr
                                                                const int64_t* __restrict__ out_off)
 {
     const int64_t total = min(capacity, out_off[T_out]) * units_per_pos;
-    constexpr int kPerThread = 8;
+    constexpr int kPerThread = kSegmentBytesPerThread / static_cast<int>(sizeof(VT));
     const int64_t chunk = 256 * kPerThread;   // consecutive units of one block and step: a table changes rarely inside
     int64_t i = -1;                            // current output table
-    int64_t seg_hi = 0, delta = 0;
+    int64_t seg_hi = 0, delta = 0;             // end of the table in units; distance to its source in units
+    auto find_table = [&](int64_t u) {
+        // largest i with out_off[i] <= o; positions only grow, so the search starts at the current table
+        const int64_t o = ONE_UNIT ? u : u / units_per_pos;   // a position is one unit for plain values
+        int64_t lo = (i < 0) ? 0 : i, hi = T_out;
+        while (hi - lo > 1) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (out_off[mid] <= o) lo = mid; else hi = mid;
+        }
+        i = lo;
+        seg_hi = out_off[i + 1] * units_per_pos;
+        const int64_t p = permute[i];
+        delta = (((p >= 0 && p < T_in) ? in_off[p] : 0) - out_off[i]) * units_per_pos;
+    };
     for (int64_t c0 = static_cast<int64_t>(blockIdx.x) * chunk; c0 < total; c0 += static_cast<int64_t>(gridDim.x) * chunk) {
-#pragma unroll 4
+        if (i < 0 || c0 >= seg_hi) find_table(c0);
+        if (c0 + chunk <= min(total, seg_hi)) {              // the same for the whole block
+            VT v[kPerThread];
+            const VT* from = src + c0 + delta + threadIdx.x;
+            VT* to = dst + c0 + threadIdx.x;
+#pragma unroll
+            for (int j = 0; j < kPerThread; ++j) v[j] = __ldg(from + j * 256);
+#pragma unroll
+            for (int j = 0; j < kPerThread; ++j) to[j * 256] = v[j];
+            continue;
+        }
+#pragma unroll 1
         for (int j = 0; j < kPerThread; ++j) {
             const int64_t u = c0 + j * 256 + threadIdx.x;
             if (u >= total) break;
-            const int64_t o = ONE_UNIT ? u : u / units_per_pos;   // a position is one unit for plain values
-            if (i < 0 || o >= seg_hi) {
-                // largest i with out_off[i] <= o; positions only grow, so the search starts at the current table
-                int64_t lo = (i < 0) ? 0 : i, hi = T_out;
-                while (hi - lo > 1) {
-                    const int64_t mid = (lo + hi) >> 1;
-                    if (out_off[mid] <= o) lo = mid; else hi = mid;
-                }
-                i = lo;
-                seg_hi = out_off[i + 1];
-                const int64_t p = permute[i];
-                delta = ((p >= 0 && p < T_in) ? in_off[p] : 0) - out_off[i];
-            }
-            dst[u] = src[u + (ONE_UNIT ? delta : delta * units_per_pos)];
+            if (u >= seg_hi) find_table(u);
+            dst[u] = src[u + delta];
         }
+        i = -1;                                               // the threads may have walked to different tables
     }
 }
 
@@ -644,7 +719,8 @@ int launch_segments(const void* src, void* dst, int64_t units_per_pos, int64_t c
 {
     const int64_t units = capacity * units_per_pos;
     if (units <= 0) return TBE_B200_OK;
-    const int64_t want = (units + 256 * 8 - 1) / (256 * 8);   // eight units per thread and step
+    const int64_t chunk = 256 * (kSegmentBytesPerThread / static_cast<int64_t>(sizeof(VT)));
+    const int64_t want = (units + chunk - 1) / chunk;
     const int64_t cap = static_cast<int64_t>(sm_count()) * 32;
     const unsigned blocks = static_cast<unsigned>(want < cap ? want : cap);
     if (units_per_pos == 1)
@@ -780,10 +856,10 @@ extern "C" int tbe_b200_complete_cumsum(const void* in, int64_t n, int index_bit
 extern "C" int64_t tbe_b200_permute_2d_sparse_scratch_bytes(int64_t T_in, int64_t T_out)
 {
     if (T_in < 0 || T_out < 0) return 0;
-    return (T_in + (T_in + 1) + (T_out + 1)) * 8;
+    return (T_in * tbe::kMaxPartials + (T_in + 1) + (T_out + 1)) * 8;
 }
 
-// Scratch layout: seg_len[T_in], in_off[T_in + 1], out_off[T_out + 1], all int64.
+// Scratch layout: the tables' partial sums [T_in * kMaxPartials], in_off[T_in + 1], out_off[T_out + 1], all int64.
 extern "C" int tbe_b200_permute_2d_sparse_offsets(const int32_t* permute, int64_t T_out, const void* lengths, int lengths_bits, int64_t T_in,
                                                   int64_t B, void* out_lengths, void* scratch, int64_t scratch_bytes, int32_t* error_flag,
                                                   tbe_b200_stream_t stream)
@@ -798,26 +874,26 @@ extern "C" int tbe_b200_permute_2d_sparse_offsets(const int32_t* permute, int64_
                     static_cast<long long>(tbe_b200_permute_2d_sparse_scratch_bytes(T_in, T_out)), static_cast<long long>(scratch_bytes));
     if (T_in > 65535 || T_out > 65535) return fail(TBE_B200_ERR_UNSUPPORTED, "permute_2d_sparse: at most 65535 tables");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int64_t* seg_len = static_cast<int64_t*>(scratch);
-    int64_t* in_off = seg_len + T_in;
+    int64_t* partials = static_cast<int64_t*>(scratch);
+    int64_t* in_off = partials + T_in * kMaxPartials;
     int64_t* out_off = in_off + T_in + 1;
-    if (cudaMemsetAsync(seg_len, 0, static_cast<size_t>(T_in) * 8, s) != cudaSuccess)
-        return fail(TBE_B200_ERR_CUDA, "permute_2d_sparse: memset failed");
-    const int64_t per_row = (B + 256 * 8 - 1) / (256 * 8);
-    const unsigned gx = static_cast<unsigned>(per_row < 64 ? per_row : 64);
-    if (lengths_bits == 32) {
-        segment_lengths_kernel<int32_t><<<dim3(gx, static_cast<unsigned>(T_in)), 256, 0, s>>>(static_cast<const int32_t*>(lengths), B, seg_len);
-    } else {
-        segment_lengths_kernel<int64_t><<<dim3(gx, static_cast<unsigned>(T_in)), 256, 0, s>>>(static_cast<const int64_t*>(lengths), B, seg_len);
-    }
-    segment_offsets_kernel<<<1, kScanThreads, 0, s>>>(seg_len, T_in, permute, T_out, in_off, out_off, error_flag);
-    if (lengths_bits == 32) {
-        permute_lengths_kernel<int32_t><<<dim3(gx, static_cast<unsigned>(T_out)), 256, 0, s>>>(static_cast<const int32_t*>(lengths), T_in, B, permute,
-                                                                                                static_cast<int32_t*>(out_lengths));
-    } else {
-        permute_lengths_kernel<int64_t><<<dim3(gx, static_cast<unsigned>(T_out)), 256, 0, s>>>(static_cast<const int64_t*>(lengths), T_in, B, permute,
-                                                                                                static_cast<int64_t*>(out_lengths));
-    }
+    const int64_t slices64 = (B + 256 * 8 - 1) / (256 * 8);                 // eight lengths per thread, at least
+    const unsigned per_table = static_cast<unsigned>(slices64 < kMaxPartials ? slices64 : kMaxPartials);
+    const unsigned slices = static_cast<unsigned>(slices64 < 64 ? slices64 : 64);
+    auto launch = [&](auto tag) {
+        using T = decltype(tag);
+        const T* len = static_cast<const T*>(lengths);
+        T* out = static_cast<T*>(out_lengths);
+        if (small_request(T_in, T_out, B)) {
+            small_offsets_and_lengths_kernel<T><<<1, kSmallThreads, 0, s>>>(len, T_in, B, permute, T_out, out, in_off, out_off, error_flag);
+            return;
+        }
+        segment_partials_kernel<T><<<dim3(per_table, static_cast<unsigned>(T_in)), 256, 0, s>>>(len, B, partials);
+        offsets_and_lengths_kernel<T><<<dim3(1 + slices, static_cast<unsigned>(T_out)), kOffsetThreads, 0, s>>>(
+            partials, static_cast<int>(per_table), len, T_in, B, permute, T_out, out, in_off, out_off, error_flag);
+    };
+    if (lengths_bits == 32) launch(int32_t{});
+    else launch(int64_t{});
     return check_launch("permute_2d_sparse_offsets");
 }
 
@@ -833,8 +909,7 @@ extern "C" int tbe_b200_permute_2d_sparse_copy(const int32_t* permute, int64_t T
     if (!values || !out_values || value_bytes <= 0) return fail(TBE_B200_ERR_INVALID_ARGUMENT, "permute_2d_sparse: values are missing");
     if (weights && (!out_weights || weight_row_bytes <= 0)) return fail(TBE_B200_ERR_INVALID_ARGUMENT, "permute_2d_sparse: weights output is missing");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const int64_t* seg_len = static_cast<const int64_t*>(scratch);
-    const int64_t* in_off = seg_len + T_in;
+    const int64_t* in_off = static_cast<const int64_t*>(scratch) + T_in * kMaxPartials;
     const int64_t* out_off = in_off + T_in + 1;
     int rc = copy_segments(values, out_values, value_bytes, out_capacity, permute, T_in, T_out, in_off, out_off, s);
     if (rc != TBE_B200_OK) return rc;
@@ -857,8 +932,7 @@ extern "C" int tbe_b200_permute_2d_sparse_copy_to_dests(const int32_t* permute, 
     if (total_hint == 0) return TBE_B200_OK;
     if (!values || value_bytes <= 0) return fail(TBE_B200_ERR_INVALID_ARGUMENT, "permute_2d_sparse_copy_to_dests: values are missing");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const int64_t* seg_len = static_cast<const int64_t*>(scratch);
-    const int64_t* in_off = seg_len + T_in;
+    const int64_t* in_off = static_cast<const int64_t*>(scratch) + T_in * kMaxPartials;
     const int64_t* out_off = in_off + T_in + 1;
     // unit of the copy: the widest that divides a value and the source address (destinations are 16-byte aligned)
     const uintptr_t a = reinterpret_cast<uintptr_t>(values);

@@ -221,7 +221,7 @@ int tbe_b200_complete_cumsum_static(const void* in, int64_t n, int index_bits, v
  *     out_lengths[i, :] = lengths[permute[i], :]
  *     out_values  = values of table permute[0], then of permute[1], ...     (weights alike)
  * Two calls, so that a caller that does not know the output size can read it in between:
- *   _offsets  fills out_lengths and the scratch: seg_len[T_in], in_off[T_in + 1], out_off[T_out + 1], all
+ *   _offsets  fills out_lengths and the scratch: partial sums, then in_off[T_in + 1], out_off[T_out + 1], all
  *             int64; out_off[T_out] (the last word) is the number of output values.
  *   _copy     moves min(out_capacity, out_off[T_out]) values of value_bytes each, and as many weight rows of
  *             weight_row_bytes (weights may be NULL), using the scratch the first call left.

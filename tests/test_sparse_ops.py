@@ -263,6 +263,30 @@ def test_permute_2d_sparse_data_shapes(shape, wcols):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("t_in,t_out,b", [(1, 1, 512), (1, 3, 513), (32, 32, 512), (33, 20, 512), (128, 128, 128), (129, 128, 4), (128, 129, 4),
+                                          (3, 2, 2048), (3, 2, 2049), (2, 5, 70000), (300, 257, 60)])
+@pytest.mark.parametrize("vname", ["int64", "int32", "float16"])
+def test_permute_2d_at_the_edges_of_its_forms(t_in, t_out, b, vname):
+    """Table counts and batches around what the one-block form takes and around the slices of the other one; table lengths
+    that fill whole copy chunks exactly, end one short of them, and are empty."""
+    import torch
+    import fbgemm_ascend_b200  # noqa: F401
+
+    rng = _rng("edges", t_in, t_out, b, vname)
+    per_chunk = 256 * 64 // np.dtype(vname).itemsize
+    lengths = rng.integers(0, 3, (t_in, b)).astype(np.int32)
+    lengths[0, :] = 0
+    lengths[0, 0] = per_chunk * 2
+    if t_in > 2:
+        lengths[1, :] = 0
+        lengths[2, 0] += per_chunk - 1
+    values = torch.from_numpy(rng.integers(0, 1000, int(lengths.sum())).astype(vname))
+    permute = rng.integers(0, t_in, t_out).astype(np.int32)
+    permute[0] = 0
+    _check_permute(torch.ops.fbgemm.permute_2D_sparse_data, permute, lengths, values, None, True)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("vname", ["int64", "float16"])
 @pytest.mark.parametrize("wname", [None, "float32"])
 def test_permute_1d_and_input1d(vname, wname):
