@@ -1495,9 +1495,14 @@ tbe_pooled_kernel(const __grid_constant__ LookupParams p)
 //
 // Row n of the output gets the dequantised row indices[n] of the table that position n belongs to (the t with
 // offsets[t*B] <= n < offsets[(t+1)*B]), zero-filled from D_t up to max_D.  A warp takes kNobagChunk consecutive
-// positions: the table is found once by binary search and then followed, and G = 32 / LPR rows are handled per
-// pass, LPR lanes per row, 16 elements per lane, with the same chunk-to-element mapping as the pooled path.
-// Nothing is accumulated, so rows go straight to registers; value = code * scale + bias in one mixed FMA.
+// positions: the table is found once by binary search and then followed.
+//
+// The output is larger than the input here, so the work is cut by OUTPUT: a lane makes one 16-byte piece (8 elements of
+// 16 bits or 4 of 32) at a time and consecutive lanes take consecutive pieces, so every store instruction writes 512
+// contiguous bytes straight from registers.  The few row bytes behind a piece are fetched with 4-byte (INT8: two)
+// loads that neighbouring lanes coalesce, the header with one more that hits L1.  Value = code * scale + bias in one mixed
+// FMA.  1.6 M rows of 128 INT8 codes to fp16 (26 tables of a million rows, 410 MB of output): 160 us with the rows put
+// together in shared memory first, 128 us this way (a copy of the same bytes: 76 us).
 
 constexpr int kNobagChunk = 64;
 
@@ -1524,52 +1529,29 @@ __device__ __noinline__ void nobag_position_bytewise(const LookupParams& p, cons
     for (int e = m.D + lane; e < max_D; e += kWarp) store_scalar(seg, e, 0.0f, p.out_ty);
 }
 
-// Four consecutive output elements of a row image in shared memory (e0 a multiple of 4).
-__device__ __forceinline__ void stage_out4(uint8_t* row_image, int e0, const float* v, int out_ty)
-{
-    if (out_ty == TBE_B200_FP32) {
-        *reinterpret_cast<float4*>(row_image + e0 * 4) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-        uint32_t h[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) h[j] = (out_ty == TBE_B200_FP16) ? f32_to_f16_bits(v[j]) : f32_to_bf16_bits(v[j]);
-        *reinterpret_cast<uint2*>(row_image + e0 * 2) = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-    }
-}
-
-constexpr int kNobagStageBytes = 2048;   // the G rows of one step: at most 512 elements of 4 bytes
-
-// `cnt` consecutive positions [n, n + cnt) of one table with aligned rows of D = 16 * units <= 512 elements.
-// A lane's 16 decoded elements start 4 (INT8) or 8 (INT4) elements before a 16-element boundary, so stored from
-// registers they are 8-byte pieces 32 bytes apart: every 32-byte sector of the output -- which is larger than the
-// input here -- is written in part by several instructions.  With a 16-byte aligned output the G rows of a step are
-// put together in the warp's `stage` area and leave as whole 16-byte pieces, consecutive from lane to lane.
-template <int TY, int LPR, typename IdxT>
-__device__ __forceinline__ void nobag_rows(const LookupParams& p, const TableMeta& m, const IdxT* indices, int64_t n, int cnt, int max_D,
-                                           int lane, uint8_t* stage)
+// `cnt` consecutive positions [n, n + cnt), cnt <= kNobagChunk, of one table with 16-byte aligned rows of D elements, D a
+// multiple of EP: EP elements are one 16-byte piece of the output.
+template <int TY, int EP>
+__device__ __forceinline__ void nobag_pieces(const LookupParams& p, const TableMeta& m, int64_t n, int cnt, int max_D, int lane)
 {
     constexpr bool kHdr = (TY == TBE_B200_INT8 || TY == TBE_B200_INT4);
-    constexpr bool k8 = (TY == TBE_B200_INT8);
-    constexpr int CH = (TY == TBE_B200_INT4) ? 8 : 16;
-    constexpr int NCH = (TY == TBE_B200_FP16) ? 2 : (TY == TBE_B200_FP32) ? 4 : 1;
-    constexpr int EPC = 16 / NCH;
-    constexpr int HS = k8 ? 4 : (TY == TBE_B200_INT4 ? 8 : 0);
-    constexpr int G = kWarp / LPR;
-    const int k = lane % LPR, g = lane / LPR;
-    const int D = m.D, nunits = D / 16;
-    const bool head_lane = kHdr && k == 0;
-    const bool active = k < nunits;
-    const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
-    const int row_out_bytes = D * esz, pieces_per_row = row_out_bytes / 16;
-    const int piece_shift = (pieces_per_row & (pieces_per_row - 1)) == 0 ? __ffs(pieces_per_row) - 1 : -1;   // power of two: no division
-    const bool staged = (reinterpret_cast<uintptr_t>(p.output) & 15) == 0 && (p.out_stride * esz) % 16 == 0;   // warp-uniform
-    // The warp's positions are narrowed and checked once (lane l holds positions l and l + 32), then taken U steps of
-    // G rows at a time: the row loads of all U steps are issued before the first row is decoded, so U * G rows per warp
-    // are in flight instead of G.
-    constexpr int U = (NCH == 1) ? 4 : (NCH == 2 ? 2 : 1);
+    // bytes and 32-bit words of a row behind one piece
+    constexpr int PB = (TY == TBE_B200_INT4) ? EP / 2 : (TY == TBE_B200_FP16) ? 2 * EP : (TY == TBE_B200_FP32) ? 4 * EP : EP;
+    constexpr int RW = (PB + 3) / 4;
+    constexpr int U = RW <= 2 ? 4 : 2;                 // pieces per lane in flight
+    const int D = m.D, width = max(D, max_D);
+    const int per_row = (width + EP - 1) / EP;         // pieces of an output row (below 8192: the division by it is exact)
+    const uint32_t inv = 0xffffffffu / static_cast<uint32_t>(per_row) + 1u;
+    const int total = cnt * per_row;
+    constexpr int esz = 16 / EP;
+    const bool vec = (reinterpret_cast<uintptr_t>(p.output) & 15) == 0 && (p.out_stride * esz) % 16 == 0;
+    char* out = static_cast<char*>(p.output) + n * p.out_stride * esz;
+    const int64_t out_row_bytes = p.out_stride * esz;
+    // The positions' row numbers, checked once: lane l holds positions l and l + 32.
     auto checked = [&](int pos) -> int32_t {
         if (pos >= cnt) return -1;
-        int64_t idx = static_cast<int64_t>(__ldg(indices + n + pos));
+        const int64_t idx = p.idx64 ? __ldg(static_cast<const int64_t*>(p.indices) + n + pos)
+                                    : static_cast<int64_t>(__ldg(static_cast<const int32_t*>(p.indices) + n + pos));
         if ((idx < -1 || idx > 0x7fffffffll) && p.error_flag) atomicOr(p.error_flag, 1);
         if (idx > 0x7fffffffll || idx < 0) return -1;
         if (static_cast<uint64_t>(idx + 1) * static_cast<uint64_t>(m.stride) > static_cast<uint64_t>(m.avail)) {
@@ -1579,145 +1561,127 @@ __device__ __forceinline__ void nobag_rows(const LookupParams& p, const TableMet
         return static_cast<int32_t>(idx);
     };
     const int32_t idx_lo = checked(lane), idx_hi = checked(lane + 32);
-    for (int r0 = 0; r0 < cnt; r0 += G * U) {
-        uint32_t words_u[U][4 * NCH];
-        uint32_t tail_u[U];
+#pragma unroll 1
+    for (int i0 = 0; i0 < total; i0 += kWarp * U) {
+        uint32_t raw[U][RW], hdr[U];
+        int row_u[U], k_u[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int pos = r0 + u * G + g;
-            const int32_t a = __shfl_sync(kFull, idx_lo, pos & 31), b = __shfl_sync(kFull, idx_hi, pos & 31);
-            const int32_t idx = pos < 32 ? a : (pos < 64 ? b : -1);
-            const bool ok = idx >= 0;
-            const uint8_t* row = m.table + static_cast<int64_t>(ok ? idx : 0) * m.stride;
+            const uint32_t i = static_cast<uint32_t>(i0 + u * kWarp + lane);
+            // (one piece per row: the reciprocal does not fit 32 bits)
+            const int row = per_row == 1 ? static_cast<int>(i) : static_cast<int>(__umulhi(i, inv));
+            const int k = static_cast<int>(i) - row * per_row;
+            const int32_t a = __shfl_sync(kFull, idx_lo, row & 31), b = __shfl_sync(kFull, idx_hi, row & 31);
+            const int32_t idx = row < 32 ? a : b;
+            row_u[u] = row;
+            k_u[u] = k;
+            hdr[u] = 0u;
 #pragma unroll
-            for (int c = 0; c < 4 * NCH; ++c) words_u[u][c] = 0u;
-            tail_u[u] = 0u;
-            if (ok && active) {
-                if constexpr (TY == TBE_B200_INT4) {
-                    const uint2 v = ldg8(row + k * 8);
-                    words_u[u][0] = v.x; words_u[u][1] = v.y;
-                } else {
+            for (int w = 0; w < RW; ++w) raw[u][w] = 0u;
+            if (row < cnt && idx >= 0 && k * EP < D) {
+                const uint8_t* base = m.table + static_cast<int64_t>(idx) * m.stride;
+                if constexpr (kHdr) hdr[u] = ldg4(base);
+                const uint8_t* q = base + (kHdr ? 4 : 0) + k * PB;
+                if constexpr (PB == 2) {
+                    raw[u][0] = __ldg(reinterpret_cast<const unsigned short*>(q));
+                } else if constexpr (PB >= 16) {
 #pragma unroll
-                    for (int c = 0; c < NCH; ++c) {
-                        const uint4 v = ldg16(row + 16 * (k + c * nunits));
-                        words_u[u][4 * c + 0] = v.x; words_u[u][4 * c + 1] = v.y; words_u[u][4 * c + 2] = v.z; words_u[u][4 * c + 3] = v.w;
+                    for (int w = 0; w < RW; w += 4) {
+                        const uint4 v = ldg16(q + 4 * w);
+                        raw[u][w] = v.x; raw[u][w + 1] = v.y; raw[u][w + 2] = v.z; raw[u][w + 3] = v.w;
                     }
+                } else if constexpr (PB == 8 && !kHdr) {
+                    const uint2 v = ldg8(q);
+                    raw[u][0] = v.x; raw[u][1] = v.y;
+                } else {                               // behind the header only 4-byte alignment is left
+#pragma unroll
+                    for (int w = 0; w < RW; ++w) raw[u][w] = ldg4(q + 4 * w);
                 }
-                if (head_lane) tail_u[u] = ldg4(row + (k8 ? D : D / 2));
             }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-        const uint32_t* words = words_u[u];
-        const uint32_t tail = tail_u[u];
-        const int pos = r0 + u * G + g;
-        const bool mine = pos < cnt;
-        float v[16];
-        if constexpr (kHdr) {
-            const uint32_t hdr = __shfl_sync(kFull, words[0], 0, LPR);   // zero for a row that is not read
-            const uint32_t w0 = head_lane ? tail : words[0];
-            const unsigned short scale_h = static_cast<unsigned short>(hdr & 0xffffu);
-            const float bias = half_bits_to_float(hdr >> 16);
+            if (row_u[u] >= cnt) continue;
+            float v[EP];
+            if constexpr (kHdr) {
+                const unsigned short scale_h = static_cast<unsigned short>(hdr[u] & 0xffffu);
+                const float bias = half_bits_to_float(hdr[u] >> 16);
 #pragma unroll
-            for (int s = 0; s < 16; ++s) v[s] = bias;
-            if (k8) {
+                for (int s = 0; s < EP; ++s) v[s] = bias;
+                if constexpr (TY == TBE_B200_INT8) {
 #pragma unroll
-                for (int i4 = 0; i4 < 4; ++i4) {
-                    const uint32_t c = (i4 == 0) ? w0 : words[i4];
-                    const uint32_t even = codes_to_half2((c & 0x00FF00FFu) | 0x64006400u, 0x64006400u);
-                    const uint32_t odd = codes_to_half2(__byte_perm(c, 0x64646464u, 0x4341), 0x64006400u);
-                    add_pair_t<false>(v[4 * i4 + 0], v[4 * i4 + 2], even, scale_h, 0.0f);
-                    add_pair_t<false>(v[4 * i4 + 1], v[4 * i4 + 3], odd, scale_h, 0.0f);
-                }
-            } else {
-#pragma unroll
-                for (int i2 = 0; i2 < 2; ++i2) {
-                    const uint32_t c = (i2 == 0) ? w0 : words[i2];
+                    for (int w = 0; w < RW; ++w) {
+                        const uint32_t c = raw[u][w];
+                        const uint32_t even = codes_to_half2((c & 0x00FF00FFu) | 0x64006400u, 0x64006400u);
+                        const uint32_t odd = codes_to_half2(__byte_perm(c, 0x64646464u, 0x4341), 0x64006400u);
+                        add_pair_t<false>(v[4 * w + 0], v[4 * w + 2], even, scale_h, 0.0f);
+                        add_pair_t<false>(v[4 * w + 1], v[4 * w + 3], odd, scale_h, 0.0f);
+                    }
+                } else {
+                    // nibble pairs (j, j + EP / 2) are brought 16 bits apart
+                    const uint32_t c = EP == 8 ? raw[u][0] : ((raw[u][0] & 0xffu) | ((raw[u][0] & 0xff00u) << 8));
                     const uint32_t y = c >> 8;
                     const uint32_t p0 = codes_to_half2((c & 0x000F000Fu) | 0x64006400u, 0x64006400u);
                     const uint32_t p1 = codes_to_half2((c & 0x00F000F0u) | 0x54005400u, 0x54005400u);
-                    const uint32_t p2 = codes_to_half2((y & 0x000F000Fu) | 0x64006400u, 0x64006400u);
-                    const uint32_t p3 = codes_to_half2((y & 0x00F000F0u) | 0x54005400u, 0x54005400u);
-                    add_pair_t<false>(v[8 * i2 + 0], v[8 * i2 + 4], p0, scale_h, 0.0f);
-                    add_pair_t<false>(v[8 * i2 + 1], v[8 * i2 + 5], p1, scale_h, 0.0f);
-                    add_pair_t<false>(v[8 * i2 + 2], v[8 * i2 + 6], p2, scale_h, 0.0f);
-                    add_pair_t<false>(v[8 * i2 + 3], v[8 * i2 + 7], p3, scale_h, 0.0f);
+                    add_pair_t<false>(v[0], v[EP / 2], p0, scale_h, 0.0f);
+                    add_pair_t<false>(v[1], v[EP / 2 + 1], p1, scale_h, 0.0f);
+                    if constexpr (EP == 8) {
+                        const uint32_t p2 = codes_to_half2((y & 0x000F000Fu) | 0x64006400u, 0x64006400u);
+                        const uint32_t p3 = codes_to_half2((y & 0x00F000F0u) | 0x54005400u, 0x54005400u);
+                        add_pair_t<false>(v[2], v[6], p2, scale_h, 0.0f);
+                        add_pair_t<false>(v[3], v[7], p3, scale_h, 0.0f);
+                    }
                 }
-            }
-        } else if constexpr (TY == TBE_B200_FP8) {
+            } else if constexpr (TY == TBE_B200_FP8) {
 #pragma unroll
-            for (int s = 0; s < 16; ++s) {
-                const uint32_t by = (words[s >> 2] >> (8 * (s & 3))) & 0xffu;
-                const float mag = __uint_as_float((by & 0x7fu) << p.fp8_shift) * p.fp8_mult;
-                v[s] = __uint_as_float(__float_as_uint(mag) | ((by & 0x80u) << 24));
-            }
-        } else if constexpr (TY == TBE_B200_FP16) {
-#pragma unroll
-            for (int s = 0; s < 16; ++s) v[s] = half_bits_to_float((words[s >> 1] >> (16 * (s & 1))) & 0xffffu);
-        } else {
-#pragma unroll
-            for (int s = 0; s < 16; ++s) v[s] = __uint_as_float(words[s]);
-        }
-        if (staged) {
-            if (active) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int slot = 4 * q;
-                    int e0;
-                    if constexpr (kHdr) e0 = (head_lane && slot < HS) ? (D - HS + slot) : (16 * k - HS + slot);
-                    else e0 = EPC * (k + (slot / EPC) * nunits) + (slot % EPC);
-                    stage_out4(stage + g * row_out_bytes, e0, &v[slot], p.out_ty);
+                for (int s = 0; s < EP; ++s) {
+                    const uint32_t by = (raw[u][s >> 2] >> (8 * (s & 3))) & 0xffu;
+                    const float mag = __uint_as_float((by & 0x7fu) << p.fp8_shift) * p.fp8_mult;
+                    v[s] = __uint_as_float(__float_as_uint(mag) | ((by & 0x80u) << 24));
                 }
-            }
-            __syncwarp();
-            for (int c = lane; c < G * pieces_per_row; c += kWarp) {
-                const int row = piece_shift >= 0 ? (c >> piece_shift) : c / pieces_per_row, piece = c - row * pieces_per_row;
-                const int rpos = r0 + u * G + row;
-                if (rpos < cnt)
-                    st_stream16(static_cast<char*>(p.output) + (n + rpos) * p.out_stride * esz + 16 * piece,
-                                *reinterpret_cast<const uint4*>(stage + row * row_out_bytes + 16 * piece));
-            }
-            __syncwarp();
-            if (mine) {
-                char* seg = static_cast<char*>(p.output) + (n + pos) * p.out_stride * esz;
-                for (int e = D + k; e < max_D; e += LPR) store_scalar(seg, e, 0.0f, p.out_ty);
-            }
-        } else if (mine) {
-            char* seg = static_cast<char*>(p.output) + (n + pos) * p.out_stride * esz;
-            const bool vec = ((reinterpret_cast<uintptr_t>(seg)) & 15) == 0;
-            if (active) {
+            } else if constexpr (TY == TBE_B200_FP16) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int slot = 4 * q;
-                    int e0;
-                    if constexpr (kHdr) e0 = (head_lane && slot < HS) ? (D - HS + slot) : (16 * k - HS + slot);
-                    else e0 = EPC * (k + (slot / EPC) * nunits) + (slot % EPC);
-                    store_out<4>(seg, e0, &v[slot], p.out_ty, vec);
-                }
+                for (int s = 0; s < EP; ++s) v[s] = half_bits_to_float((raw[u][s >> 1] >> (16 * (s & 1))) & 0xffffu);
+            } else {
+#pragma unroll
+                for (int s = 0; s < EP; ++s) v[s] = __uint_as_float(raw[u][s]);
             }
-            for (int e = D + k; e < max_D; e += LPR) store_scalar(seg, e, 0.0f, p.out_ty);
-        }
+            char* dst = out + row_u[u] * out_row_bytes + k_u[u] * 16;
+            if (vec && (k_u[u] + 1) * EP <= width) {
+                if constexpr (EP == 4) {
+                    store_out<4>(dst, 0, v, TBE_B200_FP32, true);
+                } else {
+                    uint32_t h[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (p.out_ty == TBE_B200_FP16) {
+                            const __half2 x = __floats2half2_rn(v[2 * q], v[2 * q + 1]);
+                            h[q] = *reinterpret_cast<const uint32_t*>(&x);
+                        } else {
+                            const __nv_bfloat162 x = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+                            h[q] = *reinterpret_cast<const uint32_t*>(&x);
+                        }
+                    }
+                    st_stream16(dst, make_uint4(h[0], h[1], h[2], h[3]));
+                }
+            } else {
+                for (int s = 0; s < EP && k_u[u] * EP + s < width; ++s) store_scalar(dst, s, v[s], p.out_ty);
+            }
         }
     }
 }
 
-template <int TY, typename IdxT>
-__device__ __forceinline__ void nobag_rows_by_width(const LookupParams& p, const TableMeta& m, const IdxT* indices, int64_t n, int cnt,
-                                                    int max_D, int lane, uint8_t* stage)
+template <int TY>
+__device__ __forceinline__ void nobag_pieces_by_output(const LookupParams& p, const TableMeta& m, int64_t n, int cnt, int max_D, int lane)
 {
-    const int nunits = m.D / 16;
-    if (nunits <= 4) nobag_rows<TY, 4, IdxT>(p, m, indices, n, cnt, max_D, lane, stage);
-    else if (nunits <= 8) nobag_rows<TY, 8, IdxT>(p, m, indices, n, cnt, max_D, lane, stage);
-    else if (nunits <= 16) nobag_rows<TY, 16, IdxT>(p, m, indices, n, cnt, max_D, lane, stage);
-    else nobag_rows<TY, 32, IdxT>(p, m, indices, n, cnt, max_D, lane, stage);
+    if (p.out_ty == TBE_B200_FP32) nobag_pieces<TY, 4>(p, m, n, cnt, max_D, lane);
+    else nobag_pieces<TY, 8>(p, m, n, cnt, max_D, lane);
 }
 
 template <typename IdxT>
 __global__ void __launch_bounds__(kWarpsPerBlock* kWarp)
 tbe_nobag_kernel(const __grid_constant__ LookupParams p, int64_t num_indices, int max_D)
 {
-    __shared__ __align__(16) uint8_t stage_all[kWarpsPerBlock][kNobagStageBytes];
-    uint8_t* stage = stage_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
     int64_t n = gw * kNobagChunk;
@@ -1744,15 +1708,17 @@ tbe_nobag_kernel(const __grid_constant__ LookupParams p, int64_t num_indices, in
         if (stop <= n) stop = n_end;   // offsets that do not cover every position: the last table takes the rest
         const TableMeta m = load_meta(p, t);
         const int cnt = static_cast<int>(stop - n);
-        const bool fast = m.rows_aligned && m.D > 0 && (m.D & 15) == 0 && m.D <= 512;
+        // whole pieces of 8 (16-bit output) or 4 elements; an output row of fewer than 8192 of them
+        const int ep = p.out_ty == TBE_B200_FP32 ? 4 : 8;
+        const bool fast = m.rows_aligned && m.D > 0 && m.D % ep == 0 && max(m.D, max_D) < 8191 * ep;
         bool done = fast;
         if (fast) {
             switch (m.ty) {
-                case TBE_B200_INT8: nobag_rows_by_width<TBE_B200_INT8, IdxT>(p, m, indices, n, cnt, max_D, lane, stage); break;
-                case TBE_B200_INT4: nobag_rows_by_width<TBE_B200_INT4, IdxT>(p, m, indices, n, cnt, max_D, lane, stage); break;
-                case TBE_B200_FP8: nobag_rows_by_width<TBE_B200_FP8, IdxT>(p, m, indices, n, cnt, max_D, lane, stage); break;
-                case TBE_B200_FP16: nobag_rows_by_width<TBE_B200_FP16, IdxT>(p, m, indices, n, cnt, max_D, lane, stage); break;
-                case TBE_B200_FP32: nobag_rows_by_width<TBE_B200_FP32, IdxT>(p, m, indices, n, cnt, max_D, lane, stage); break;
+                case TBE_B200_INT8: nobag_pieces_by_output<TBE_B200_INT8>(p, m, n, cnt, max_D, lane); break;
+                case TBE_B200_INT4: nobag_pieces_by_output<TBE_B200_INT4>(p, m, n, cnt, max_D, lane); break;
+                case TBE_B200_FP8: nobag_pieces_by_output<TBE_B200_FP8>(p, m, n, cnt, max_D, lane); break;
+                case TBE_B200_FP16: nobag_pieces_by_output<TBE_B200_FP16>(p, m, n, cnt, max_D, lane); break;
+                case TBE_B200_FP32: nobag_pieces_by_output<TBE_B200_FP32>(p, m, n, cnt, max_D, lane); break;
                 default: done = false; break;
             }
         }

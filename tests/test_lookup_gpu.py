@@ -335,3 +335,16 @@ def test_bags_that_straddle_lane_group_ranges(weights_ty, D, weighted):
         c = make_case(rng, [weights_ty] * 3, [D] * 3, [300, 50, 1000], B, np.asarray(lens), np.int64, weighted, prune_frac=0.01)
         for pooling, out_ty in ((O.SUM, O.FP16), (O.MEAN, O.FP32)):
             run(c, pooling, out_ty, f"straddle B={B}")
+
+
+@pytest.mark.parametrize("weights_ty,dims", [(O.INT8, [4, 12, 8, 40]), (O.INT4, [8, 40, 24, 136]), (O.FP16, [8, 20, 2, 40]), (O.FP8, [4, 24, 8, 100]),
+                                             (O.FP32, [3, 4, 20, 8])])
+@pytest.mark.parametrize("out_ty", [O.FP32, O.FP16, O.BF16])
+def test_sequence_rows_of_any_width(weights_ty, dims, out_ty):
+    """Sequence mode with tables of several widths (the narrower ones zero-filled), widths that are not whole 16-byte pieces of
+    the output, output rows that are not 16-byte aligned, pruned rows, and counts around the 64 positions of a warp."""
+    rng = np.random.default_rng(seed_of("sequence", weights_ty, dims))
+    lens = np.array([0, 63, 64, 65, 1, 0, 130, 5])
+    for ds in (dims, dims[:2]):
+        c = make_case(rng, [weights_ty] * len(ds), ds, [70] * len(ds), 2, lens[:2 * len(ds)], np.int64, False, prune_frac=0.05)
+        run(c, O.NONE, out_ty, f"sequence dims={ds}")
