@@ -80,6 +80,24 @@ def test_random_dims_bit_exact(dtype, aligned, B):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("dims", [[20, 36, 100, 4], [4, 12, 36], [2, 6, 10, 14], [1, 3, 5, 2, 7]])
+@pytest.mark.parametrize("B", [1, 7, 8, 9, 100])
+def test_pieces_of_every_width(dtype, dims, B):
+    """Features whose widths are multiples of 4, 2 and 1 elements, repeated until vectors straddle features in every way, in rows
+    that are 16-, 8-, 4- and 2-byte aligned (one feature more or less changes the row's width)."""
+    import fbgemm_ascend_b200  # noqa: F401
+    for T in (11, 12, 13):
+        d = (dims * 13)[:T]
+        perm = list(range(T))
+        random.Random(T + B).shuffle(perm)
+        off, p, inv_off, inv_p = lists(d, perm)
+        x = torch.randn(B, sum(d), device="cuda").to(dtype)
+        y = torch.ops.fbgemm.permute_pooled_embs(x, off, p, inv_off, inv_p)
+        parts = torch.split(x, d, 1)
+        assert torch.equal(y, torch.cat([parts[i] for i in perm], 1))
+
+
 def test_three_dim_input_and_validation_errors():
     import fbgemm_ascend_b200  # noqa: F401
     off, p, inv_off, inv_p = lists([8, 8], [1, 0])
