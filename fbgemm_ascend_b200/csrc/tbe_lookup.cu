@@ -15,8 +15,8 @@
 //     and accumulated in fp32.  INT8/INT4 rows start with a 4-byte header, which shifts the payload off the
 //     16-byte grid; the lane that reads the header chunk has 4 / 8 free slots, which take the row's last
 //     elements, so D = 16*LPR rows keep every lane busy with exactly 16 elements;
-//   * other aligned shapes (pool_bag; only in the build of the kernel for wide tables): one warp per bag, cp.async
-//     staging in chunks, cross-group reduce-scatter;
+//   * aligned rows of the same types and any other D that is a multiple of 4 (pool_run_steps): a warp sums its bags one after
+//     the other, eight rows per step, every unit of a row by four lanes;
 //   * anything else (row_alignment 1, odd D, INT2 or BF16 rows, unaligned tables): a byte-wise path.
 // Sequence mode (pooling NONE): tbe_nobag_kernel, 64 consecutive positions per warp.
 #include <stdarg.h>
@@ -114,27 +114,10 @@ __device__ __forceinline__ void store_out(void* seg, int e0, const float* v, int
     }
 }
 
-// ---- per-type row access ---------------------------------------------------
-//
-// Every lane owns 16 accumulator "slots".  A path says which bytes a lane fetches
-// for a row (issue), how the fetched bytes add into the slots (accum), and which
-// element of the row a slot stands for (elem).  `unit` is the lane's position
-// among the 16-slot units of the row: unit = block * LPR + k.
-//
-// Rows are fetched with cp.async straight into shared memory, never through
-// registers: each lane has private staging slots (one per pass of a chunk, two
-// chunks deep), so the rows of two chunks are in flight per warp while the
-// accumulators and addresses are all the registers a lane needs.  A lane reads
-// back only what it fetched itself, so no warp barrier is involved.
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-// 16-byte asynchronous copy global -> shared, L2 only; `bytes` = 16, or 0 to write zeros without reading.
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-// The same through L1 (the line stays cached for the rows that are fetched again and again).
+// 16-byte asynchronous copy global -> shared through L1 (the line stays cached for the rows that are fetched again and
+// again); `bytes` = 16, or 0 to write zeros without reading.
 __device__ __forceinline__ void cp_async16_ca(uint32_t dst, const void* src, int bytes)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -196,12 +179,6 @@ __device__ __forceinline__ uint32_t lds4(uint32_t a)
 // single rounding, as an fp32 FMA would.  With per-sample weights the scale is no longer an fp16
 // value; the codes are then widened to fp32 and an fp32 FMA with w * scale is used.
 
-// d = a(fp16) * b(fp16) + d(fp32), one rounding.  a, b: fp16 bit patterns in the low 16 bits.
-__device__ __forceinline__ void mixed_fma(float& d, uint32_t a, uint32_t b)
-{
-    asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(d) : "h"(static_cast<unsigned short>(a)), "h"(static_cast<unsigned short>(b)));
-}
-
 // Two exact fp16 values (as a half2 bit pattern) from two codes already or'ed into the mantissas of
 // the half2 `magic` (0x6400: 1024, 0x5400: 64 with the code in mantissa bits 4..7).
 __device__ __forceinline__ uint32_t codes_to_half2(uint32_t packed, uint32_t magic)
@@ -211,19 +188,6 @@ __device__ __forceinline__ uint32_t codes_to_half2(uint32_t packed, uint32_t mag
 }
 
 // acc[0..1] += pair (half2 bits) * scale: mixed FMA with the fp16 scale, or fp32 FMA with `ws`.
-__device__ __forceinline__ void add_pair(float& a0, float& a1, uint32_t pair, uint32_t scale_h, float ws, bool weighted)
-{
-    if (!weighted) {
-        mixed_fma(a0, pair & 0xffffu, scale_h);
-        mixed_fma(a1, pair >> 16, scale_h);
-    } else {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&pair));
-        a0 = fmaf(f.x, ws, a0);
-        a1 = fmaf(f.y, ws, a1);
-    }
-}
-
-// The same with the choice made at compile time and the two halves split inside one asm block.
 template <bool WEIGHTED>
 __device__ __forceinline__ void add_pair_t(float& a0, float& a1, uint32_t pair, unsigned short scale_h, float ws)
 {
@@ -236,428 +200,6 @@ __device__ __forceinline__ void add_pair_t(float& a0, float& a1, uint32_t pair, 
         a0 = fmaf(f.x, ws, a0);
         a1 = fmaf(f.y, ws, a1);
     }
-}
-
-// Staging memory of one warp: two chunk buffers of kChunkBytes (a lane's slot for pass u is at
-// (u*32 + lane) * slot_bytes) and, for header types, one 4-byte side slot per (buffer, pass, lane).
-constexpr int kChunkBytes = 2048;
-constexpr int kMaxPasses = 8;
-constexpr int kSideBytes = 2 * kMaxPasses * kWarp * 4;
-constexpr int kWarpSmemBytes = 2 * kChunkBytes + kSideBytes;
-
-struct LaneCtx {
-    int unit;        // 16-slot unit handled by this lane in the current block
-    int D;           // elements per row
-    int k;           // lane index within its row group
-    bool active;     // this unit exists in the row
-    bool wrap;       // INT8/INT4 header lane that also takes the row's tail
-    bool first_blk;  // block 0: the header is the first word of unit 0
-    bool weighted;   // per-sample weights are in use
-    uint32_t fp8_shift;
-    float fp8_mult;
-};
-
-template <int TY>
-struct Path;
-
-template <>
-struct Path<TBE_B200_INT8> {
-    static constexpr bool kHasHeader = true;
-    static constexpr int kSlotBytes = 16;
-    static constexpr int kPasses = 4;   // passes per chunk (x 32 lanes x 16 B = 2 KB)
-    // 16-byte chunks of the row: chunk c covers elements [16c - 4, 16c + 12).
-    static __device__ __forceinline__ int units(int D, bool wrap) { return wrap ? D / 16 : (D + 4 + 15) / 16; }
-    static __device__ __forceinline__ bool can_wrap(int D) { return (D & 15) == 0; }
-    // The side slot of the header lane gets the row's tail (elements D-4 .. D-1) when the row
-    // wraps, and the header itself in the later blocks of a wide row.
-    template <int LPR>
-    static __device__ __forceinline__ void issue(uint32_t slot, uint32_t side, const uint8_t* row, const uint8_t* safe,
-                                                 const LaneCtx& cx, bool ok)
-    {
-        if (cx.active) cp_async16(slot, ok ? row + cx.unit * 16 : safe, ok ? 16 : 0);
-        if (cx.k == 0 && (cx.wrap || !cx.first_blk)) cp_async4(side, ok ? row + (cx.wrap ? cx.D : 0) : safe, ok ? 4 : 0);
-    }
-    template <int LPR>
-    static __device__ __forceinline__ void accum(uint32_t slot, uint32_t side, const LaneCtx& cx, float w, float (&acc)[16],
-                                                 float& bias_acc)
-    {
-        uint4 v = cx.active ? lds16(slot) : make_uint4(0u, 0u, 0u, 0u);
-        uint32_t hdr = v.x;
-        if (cx.k == 0 && (cx.wrap || !cx.first_blk)) {
-            const uint32_t s = lds4(side);
-            if (cx.wrap) v.x = s; else hdr = s;
-        }
-        hdr = __shfl_sync(kFull, hdr, 0, LPR);
-        // A row that must not be added has zero-filled data and header, so its scale and bias are 0.
-        const uint32_t scale_h = hdr & 0xffffu;
-        const float ws = half_bits_to_float(scale_h) * w;
-        bias_acc = fmaf(half_bits_to_float(hdr >> 16), cx.weighted ? w : 1.0f, bias_acc);
-        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            // bytes (q0, 0x64, q1, 0x64) = half2(1024 + q0, 1024 + q1)
-            const uint32_t lo = codes_to_half2(__byte_perm(words[i], 0x64646464u, 0x4140), 0x64006400u);
-            const uint32_t hi = codes_to_half2(__byte_perm(words[i], 0x64646464u, 0x4342), 0x64006400u);
-            add_pair(acc[4 * i + 0], acc[4 * i + 1], lo, scale_h, ws, cx.weighted);
-            add_pair(acc[4 * i + 2], acc[4 * i + 3], hi, scale_h, ws, cx.weighted);
-        }
-    }
-    template <int LPR>
-    static __device__ __forceinline__ int elem(const LaneCtx& cx, int slot)
-    {
-        if (cx.wrap && slot < 4) return cx.D - 4 + slot;
-        return 16 * cx.unit - 4 + slot;
-    }
-};
-
-template <>
-struct Path<TBE_B200_INT4> {
-    static constexpr bool kHasHeader = true;
-    static constexpr int kSlotBytes = 8;
-    static constexpr int kPasses = 8;   // x 32 lanes x 8 B = 2 KB
-    // 8-byte chunks: chunk c covers elements [16c - 8, 16c + 8).
-    static __device__ __forceinline__ int units(int D, bool wrap) { return wrap ? D / 16 : (D / 2 + 4 + 7) / 8; }
-    static __device__ __forceinline__ bool can_wrap(int D) { return (D & 15) == 0; }
-    template <int LPR>
-    static __device__ __forceinline__ void issue(uint32_t slot, uint32_t side, const uint8_t* row, const uint8_t* safe,
-                                                 const LaneCtx& cx, bool ok)
-    {
-        if (cx.active) cp_async8(slot, ok ? row + cx.unit * 8 : safe, ok ? 8 : 0);
-        if (cx.k == 0 && (cx.wrap || !cx.first_blk)) cp_async4(side, ok ? row + (cx.wrap ? cx.D / 2 : 0) : safe, ok ? 4 : 0);
-    }
-    template <int LPR>
-    static __device__ __forceinline__ void accum(uint32_t slot, uint32_t side, const LaneCtx& cx, float w, float (&acc)[16],
-                                                 float& bias_acc)
-    {
-        uint2 v = cx.active ? lds8(slot) : make_uint2(0u, 0u);
-        uint32_t hdr = v.x;
-        if (cx.k == 0 && (cx.wrap || !cx.first_blk)) {
-            const uint32_t s = lds4(side);
-            if (cx.wrap) v.x = s; else hdr = s;
-        }
-        hdr = __shfl_sync(kFull, hdr, 0, LPR);
-        const uint32_t scale_h = hdr & 0xffffu;
-        const float ws = half_bits_to_float(scale_h) * w;
-        bias_acc = fmaf(half_bits_to_float(hdr >> 16), cx.weighted ? w : 1.0f, bias_acc);
-        const uint32_t words[2] = {v.x, v.y};
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            // nibble pairs (j, j + 4) sit 16 bits apart: mask them into two half mantissas at once.
-            // 0x6400 | n = 1024 + n; 0x5400 | (n << 4) = 64 + n.
-            const uint32_t x = words[i], y = words[i] >> 8;
-            const uint32_t p0 = codes_to_half2((x & 0x000F000Fu) | 0x64006400u, 0x64006400u);   // nibbles 0, 4
-            const uint32_t p1 = codes_to_half2((x & 0x00F000F0u) | 0x54005400u, 0x54005400u);   // nibbles 1, 5
-            const uint32_t p2 = codes_to_half2((y & 0x000F000Fu) | 0x64006400u, 0x64006400u);   // nibbles 2, 6
-            const uint32_t p3 = codes_to_half2((y & 0x00F000F0u) | 0x54005400u, 0x54005400u);   // nibbles 3, 7
-            add_pair(acc[8 * i + 0], acc[8 * i + 4], p0, scale_h, ws, cx.weighted);
-            add_pair(acc[8 * i + 1], acc[8 * i + 5], p1, scale_h, ws, cx.weighted);
-            add_pair(acc[8 * i + 2], acc[8 * i + 6], p2, scale_h, ws, cx.weighted);
-            add_pair(acc[8 * i + 3], acc[8 * i + 7], p3, scale_h, ws, cx.weighted);
-        }
-    }
-    template <int LPR>
-    static __device__ __forceinline__ int elem(const LaneCtx& cx, int slot)
-    {
-        if (cx.wrap && slot < 8) return cx.D - 8 + slot;
-        return 16 * cx.unit - 8 + slot;
-    }
-};
-
-template <>
-struct Path<TBE_B200_FP8> {
-    static constexpr bool kHasHeader = false;
-    static constexpr int kSlotBytes = 16;
-    static constexpr int kPasses = 4;
-    static __device__ __forceinline__ int units(int D, bool) { return (D + 15) / 16; }
-    static __device__ __forceinline__ bool can_wrap(int) { return false; }
-    template <int LPR>
-    static __device__ __forceinline__ void issue(uint32_t slot, uint32_t, const uint8_t* row, const uint8_t* safe,
-                                                 const LaneCtx& cx, bool ok)
-    {
-        if (cx.active) cp_async16(slot, ok ? row + cx.unit * 16 : safe, ok ? 16 : 0);
-    }
-    // Byte -> fp32 by bit placement: ((b & 0x7f) << (16 + ebits)) as a float, times
-    // 2^(127 - bias), sign bit or'ed in (reference: c310/op_kernel/common.h:120-167).
-    template <int LPR>
-    static __device__ __forceinline__ void accum(uint32_t slot, uint32_t, const LaneCtx& cx, float w, float (&acc)[16], float&)
-    {
-        const uint4 v = cx.active ? lds16(slot) : make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t b = (words[i] >> (8 * j)) & 0xffu;
-                const float mag = __uint_as_float((b & 0x7fu) << cx.fp8_shift) * cx.fp8_mult;
-                const float val = __uint_as_float(__float_as_uint(mag) | ((b & 0x80u) << 24));
-                acc[4 * i + j] = fmaf(w, val, acc[4 * i + j]);
-            }
-        }
-    }
-    template <int LPR>
-    static __device__ __forceinline__ int elem(const LaneCtx& cx, int slot) { return 16 * cx.unit + slot; }
-};
-
-template <>
-struct Path<TBE_B200_FP16> {
-    static constexpr bool kHasHeader = false;
-    static constexpr int kSlotBytes = 32;
-    static constexpr int kPasses = 2;
-    // A unit is two 16-byte chunks LPR chunks apart, so that one copy instruction of a group covers
-    // LPR*16 contiguous bytes: with blk = unit / LPR and k = unit % LPR, chunk_a = 2*blk*LPR + k,
-    // chunk_b = chunk_a + LPR; a chunk is 8 elements.  Bounds are checked per chunk.
-    static __device__ __forceinline__ int units(int D, bool) { return (D + 15) / 16; }
-    static __device__ __forceinline__ bool can_wrap(int) { return false; }
-    template <int LPR>
-    static __device__ __forceinline__ int chunk_a(int unit) { return 2 * (unit / LPR) * LPR + (unit % LPR); }
-    template <int LPR>
-    static __device__ __forceinline__ void issue(uint32_t slot, uint32_t, const uint8_t* row, const uint8_t* safe,
-                                                 const LaneCtx& cx, bool ok)
-    {
-        const int ca = chunk_a<LPR>(cx.unit);
-        if (ca * 8 < cx.D) cp_async16(slot, ok ? row + ca * 16 : safe, ok ? 16 : 0);
-        if ((ca + LPR) * 8 < cx.D) cp_async16(slot + 16, ok ? row + (ca + LPR) * 16 : safe, ok ? 16 : 0);
-    }
-    template <int LPR>
-    static __device__ __forceinline__ void accum(uint32_t slot, uint32_t, const LaneCtx& cx, float w, float (&acc)[16], float&)
-    {
-        const int ca = chunk_a<LPR>(cx.unit);
-        const uint4 a = (ca * 8 < cx.D) ? lds16(slot) : make_uint4(0u, 0u, 0u, 0u);
-        const uint4 b = ((ca + LPR) * 8 < cx.D) ? lds16(slot + 16) : make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t words[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        // unweighted: value * 1.0 + acc in one mixed FMA (rows not to be added are zero-filled)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) add_pair(acc[2 * i], acc[2 * i + 1], words[i], 0x3c00u, w, cx.weighted);
-    }
-    template <int LPR>
-    static __device__ __forceinline__ int elem(const LaneCtx& cx, int slot)
-    {
-        const int ca = chunk_a<LPR>(cx.unit);
-        return slot < 8 ? 8 * ca + slot : 8 * (ca + LPR) + slot - 8;
-    }
-};
-
-template <>
-struct Path<TBE_B200_FP32> {
-    static constexpr bool kHasHeader = false;
-    static constexpr int kSlotBytes = 64;
-    static constexpr int kPasses = 1;
-    // A unit is four 16-byte chunks, LPR chunks apart: chunk_m = 4*blk*LPR + m*LPR + k.
-    static __device__ __forceinline__ int units(int D, bool) { return (D + 15) / 16; }
-    static __device__ __forceinline__ bool can_wrap(int) { return false; }
-    template <int LPR>
-    static __device__ __forceinline__ int chunk0(int unit) { return 4 * (unit / LPR) * LPR + (unit % LPR); }
-    template <int LPR>
-    static __device__ __forceinline__ void issue(uint32_t slot, uint32_t, const uint8_t* row, const uint8_t* safe,
-                                                 const LaneCtx& cx, bool ok)
-    {
-        const int c0 = chunk0<LPR>(cx.unit);
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-            if ((c0 + m * LPR) * 4 < cx.D) cp_async16(slot + 16 * m, ok ? row + (c0 + m * LPR) * 16 : safe, ok ? 16 : 0);
-    }
-    template <int LPR>
-    static __device__ __forceinline__ void accum(uint32_t slot, uint32_t, const LaneCtx& cx, float w, float (&acc)[16], float&)
-    {
-        const int c0 = chunk0<LPR>(cx.unit);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const uint4 v = ((c0 + m * LPR) * 4 < cx.D) ? lds16(slot + 16 * m) : make_uint4(0u, 0u, 0u, 0u);
-            acc[4 * m + 0] = fmaf(w, __uint_as_float(v.x), acc[4 * m + 0]);
-            acc[4 * m + 1] = fmaf(w, __uint_as_float(v.y), acc[4 * m + 1]);
-            acc[4 * m + 2] = fmaf(w, __uint_as_float(v.z), acc[4 * m + 2]);
-            acc[4 * m + 3] = fmaf(w, __uint_as_float(v.w), acc[4 * m + 3]);
-        }
-    }
-    template <int LPR>
-    static __device__ __forceinline__ int elem(const LaneCtx& cx, int slot)
-    {
-        return 4 * (chunk0<LPR>(cx.unit) + (slot >> 2) * LPR) + (slot & 3);
-    }
-};
-
-// One halving step of the cross-group reduce-scatter: lanes `dist` apart swap the
-// half of their N live values that the other one keeps.
-template <int N>
-__device__ __forceinline__ void halve(float (&a)[16], int dist, bool upper)
-{
-#pragma unroll
-    for (int j = 0; j < N / 2; ++j) {
-        const float send = upper ? a[j] : a[j + N / 2];
-        const float keep = upper ? a[j + N / 2] : a[j];
-        a[j] = keep + __shfl_xor_sync(kFull, send, dist);
-    }
-}
-
-struct BagInfo {
-    const uint8_t* table;   // first row of the table
-    int64_t stride;         // bytes per row
-    int64_t start;          // first position of the bag in indices
-    int L;                  // rows in the bag
-    int D;
-    void* seg;              // output address of element 0 of the bag
-    float mean_mul;         // 1/L for MEAN, else 1
-    bool seg_aligned;       // seg is 16-byte aligned
-    int64_t avail;          // bytes of the table: a row that would end past them is skipped
-};
-
-// Up to 32 consecutive indices and weights of a bag, one per lane.  Indices are narrowed to 32 bits:
-// a row number outside [-1, 2^31) is reported through the error flag and treated as -1 (skipped).
-struct BagHead {
-    int32_t idx;   // -1 beyond the bag
-    float w;
-};
-
-template <typename IdxT>
-__device__ __forceinline__ BagHead load_batch(const IdxT* indices, const float* pw, int n, int lane, int32_t* error_flag,
-                                              int64_t stride, int64_t avail)
-{
-    BagHead h;
-    h.idx = -1;
-    h.w = 1.0f;
-    if (lane < n) {
-        const int64_t v = static_cast<int64_t>(__ldg(indices + lane));
-        const bool bad = (v < -1) || (v > 0x7fffffffll);
-        const bool past = !bad && v >= 0 && static_cast<uint64_t>(v + 1) * static_cast<uint64_t>(stride) > static_cast<uint64_t>(avail);
-        h.idx = (bad || past) ? -1 : static_cast<int32_t>(v);
-        if ((bad || past) && error_flag) atomicOr(error_flag, bad ? 1 : 4);
-        if (pw) h.w = __ldg(pw + lane);
-    }
-    return h;
-}
-
-// Pools one bag whose rows are 16-byte aligned with a 16-byte-multiple stride.
-// `head` holds the bag's first 32 indices/weights; `wsm` is the warp's staging memory.
-template <int TY, int LPR, typename IdxT>
-__device__ __forceinline__ void pool_bag(const LookupParams& p, const BagInfo& bag, const BagHead& head, int lane,
-                                         uint32_t wsm)
-{
-    using P = Path<TY>;
-    constexpr int RPI = kWarp / LPR;                                   // rows per pass of the warp
-    constexpr int UC = (P::kPasses < kWarp / RPI) ? P::kPasses : (kWarp / RPI);   // passes per chunk
-    constexpr int RC = UC * RPI;                                       // rows per chunk (divides 32)
-    constexpr int NF = 16 / RPI;                                       // finished slots per lane after the reduce-scatter
-    static_assert(UC * kWarp * P::kSlotBytes <= kChunkBytes && UC <= kMaxPasses, "chunk does not fit its buffer");
-    const int k = lane % LPR;
-    const int g = lane / LPR;
-    const IdxT* indices = static_cast<const IdxT*>(p.indices) + bag.start;
-    const float* pw = p.pw ? p.pw + bag.start : nullptr;
-    const bool wrap_row = P::can_wrap(bag.D);
-    const int nunits = P::units(bag.D, wrap_row);
-    const int nchunks = (bag.L + RC - 1) / RC;
-    const uint32_t slot0 = wsm + lane * P::kSlotBytes;
-    const uint32_t side0 = wsm + 2 * kChunkBytes + g * 4;
-
-    for (int ublk = 0; ublk < nunits; ublk += LPR) {
-        LaneCtx cx;
-        cx.unit = ublk + k;
-        cx.D = bag.D;
-        cx.k = k;
-        // FP16/FP32 units interleave their chunks, so those paths bound-check per chunk instead.
-        cx.active = (TY == TBE_B200_FP16 || TY == TBE_B200_FP32) ? true : (cx.unit < nunits);
-        cx.first_blk = (ublk == 0);
-        cx.wrap = wrap_row && cx.unit == 0;
-        cx.weighted = p.pw != nullptr;
-        cx.fp8_shift = p.fp8_shift;
-        cx.fp8_mult = p.fp8_mult;
-
-        float acc[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] = 0.0f;
-        float bias_acc = 0.0f;
-
-        // The 32 indices the lanes currently hold cover rows [batch0, batch0 + 32) of the bag.
-        int batch0 = 0;
-        int32_t my_idx = head.idx;
-        float my_w = head.w;
-        float w_buf0 = 0.0f, w_buf1 = 0.0f;   // per staging buffer: weight of row (chunk start + lane), 0 if not to be added
-
-        auto issue_chunk = [&](int c) {
-            const int row0 = c * RC;
-            if (row0 >= batch0 + kWarp) {
-                batch0 += kWarp;
-                const BagHead nb = load_batch<IdxT>(indices + batch0, pw ? pw + batch0 : nullptr, bag.L - batch0, lane,
-                                                    cx.first_blk ? p.error_flag : nullptr, bag.stride, bag.avail);
-                my_idx = nb.idx;
-                my_w = nb.w;
-            }
-            const uint32_t slot = slot0 + (c & 1) * kChunkBytes;
-            const uint32_t side = side0 + (c & 1) * (kMaxPasses * 16 * 4);
-            const int rel0 = row0 - batch0;   // position of the chunk's first row among the 32 held indices
-#pragma unroll 1
-            for (int u = 0; u < UC; ++u) {
-                const int r = rel0 + u * RPI + g;
-                const int32_t idx = __shfl_sync(kFull, my_idx, r & 31);
-                const bool ok = (row0 + u * RPI + g < bag.L) && (idx >= 0);
-                P::template issue<LPR>(slot + u * kWarp * P::kSlotBytes, side + u * 16 * 4,
-                                       bag.table + static_cast<int64_t>(idx) * bag.stride, bag.table, cx, ok);
-            }
-            cp_async_commit();
-            if (cx.weighted) {
-                // weight of row (row0 + lane) for the lanes that stand for a row of this chunk
-                const int32_t li = __shfl_sync(kFull, my_idx, (rel0 + lane) & 31);
-                float lw = __shfl_sync(kFull, my_w, (rel0 + lane) & 31);
-                if (lane >= RC || row0 + lane >= bag.L || li < 0) lw = 0.0f;
-                if (c & 1) w_buf1 = lw; else w_buf0 = lw;
-            }
-        };
-
-        if (nchunks > 0) issue_chunk(0);
-        if (nchunks > 1) issue_chunk(1);
-        for (int c = 0; c < nchunks; ++c) {
-            if (c + 1 < nchunks) cp_async_wait<1>(); else cp_async_wait<0>();
-            const uint32_t slot = slot0 + (c & 1) * kChunkBytes;
-            const uint32_t side = side0 + (c & 1) * (kMaxPasses * 16 * 4);
-            const float wb = (c & 1) ? w_buf1 : w_buf0;
-#pragma unroll 1
-            for (int u = 0; u < UC; ++u) {
-                // Unweighted: rows that are not to be added are zero-filled, so every row can use weight 1.
-                const float w = cx.weighted ? __shfl_sync(kFull, wb, u * RPI + g) : 1.0f;
-                P::template accum<LPR>(slot + u * kWarp * P::kSlotBytes, side + u * 16 * 4, cx, w, acc, bias_acc);
-            }
-            if (c + 2 < nchunks) issue_chunk(c + 2);
-        }
-
-        // Combine the RPI groups: after this every lane holds NF finished slots,
-        // slots [slot_base, slot_base + NF) of its unit.
-        int slot_base = 0;
-        if constexpr (RPI >= 2) { const bool up = (lane >> 4) & 1; halve<16>(acc, 16, up); slot_base += up ? 8 : 0; }
-        if constexpr (RPI >= 4) { const bool up = (lane >> 3) & 1; halve<8>(acc, 8, up); slot_base += up ? 4 : 0; }
-        if constexpr (RPI >= 8) { const bool up = (lane >> 2) & 1; halve<4>(acc, 4, up); slot_base += up ? 2 : 0; }
-        if constexpr (RPI >= 16) { const bool up = (lane >> 1) & 1; halve<2>(acc, 2, up); slot_base += up ? 1 : 0; }
-        if constexpr (P::kHasHeader) {
-#pragma unroll
-            for (int d = LPR; d < kWarp; d <<= 1) bias_acc += __shfl_xor_sync(kFull, bias_acc, d);
-        }
-
-        if (cx.active) {
-            constexpr int W = NF >= 4 ? 4 : NF;   // elements per store
-#pragma unroll
-            for (int q = 0; q < NF / W; ++q) {
-                const int slot = slot_base + q * W;
-                const int e0 = P::template elem<LPR>(cx, slot);
-                if (e0 >= 0 && e0 < bag.D) {
-                    float v[W];
-#pragma unroll
-                    for (int j = 0; j < W; ++j) v[j] = (acc[q * W + j] + bias_acc) * bag.mean_mul;
-                    store_out<W>(bag.seg, e0, v, p.out_ty, bag.seg_aligned);
-                }
-            }
-        }
-    }
-}
-
-template <int TY, typename IdxT>
-__device__ __forceinline__ void pool_bag_by_width(const LookupParams& p, const BagInfo& bag, const BagHead& head, int lane,
-                                                  uint32_t wsm)
-{
-    const bool wrap = Path<TY>::can_wrap(bag.D);
-    const int nunits = Path<TY>::units(bag.D, wrap);
-    if (nunits <= 2) pool_bag<TY, 2, IdxT>(p, bag, head, lane, wsm);
-    else if (nunits <= 4) pool_bag<TY, 4, IdxT>(p, bag, head, lane, wsm);
-    else if (nunits <= 8) pool_bag<TY, 8, IdxT>(p, bag, head, lane, wsm);
-    else if (nunits <= 16) pool_bag<TY, 16, IdxT>(p, bag, head, lane, wsm);
-    else pool_bag<TY, 32, IdxT>(p, bag, head, lane, wsm);
 }
 
 // Description of the table a bag belongs to; reloaded only when the warp moves on to another table.
@@ -778,9 +320,6 @@ __device__ __noinline__ void pool_bag_bytewise(const IdxT* indices, const float*
 }
 
 // ---- the common shapes: rows streamed through a shared-memory ring, groups of lanes -----------------
-
-// Zeros that stand in for a row that must not be added: zero payload, and for INT8 / INT4 a zero header (scale 0, bias 0).
-__device__ __align__(16) const uint8_t g_zero_row[2048] = {0};
 
 // Read-once streams (indices, per-sample weights): not kept in L1.
 __device__ __forceinline__ int32_t ld_once32(const void* p) { return ld_stream(static_cast<const int32_t*>(p)); }
@@ -937,7 +476,7 @@ __host__ __device__ constexpr int min3(int a, int b, int c) { return a < b ? (a 
 // 32 rows, which keeps the partial sums small enough for the extra term not to cost precision that a 16-bit
 // result could show.
 template <int TY, int LPR, int EPL, bool WEIGHTED, bool FOLD>
-__device__ __noinline__ void pool_run_stream(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
+__device__ __forceinline__ void pool_run_stream(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
                                              uint32_t wsm)
 {
     static_assert(!FOLD || (TY == TBE_B200_INT8 && !WEIGHTED), "the folded form is for unweighted INT8 pooling");
@@ -968,7 +507,6 @@ __device__ __noinline__ void pool_run_stream(const LookupParams& p, const TableM
     const uint8_t* lane_base = m.table + k * CH;
     const uint32_t tail_off = k8 ? D : D / 2;          // header lane (k = 0): where the row's last HS elements are
     const uint32_t chunk_step = static_cast<uint32_t>(nunits) * CH;    // distance between a lane's chunks
-    const uint8_t* zero_base = g_zero_row + k * 16;
     const bool idx64 = p.idx64 != 0;
     const int isz = idx64 ? 8 : 4;
     const uint32_t sm_rel = wsm + kPartBytes;
@@ -1028,14 +566,14 @@ __device__ __noinline__ void pool_run_stream(const LookupParams& p, const TableM
     (void)scale_acc;
     (void)since_fold;
 
+    char* const out0 = static_cast<char*>(p.output) + (b0 * p.out_stride + m.col) * ((p.out_ty == TBE_B200_FP32) ? 4 : 2);   // bag 0 of the run
     // Stores the finished bag `bag` of L rows (acc + bias_acc, times 1/L for MEAN).  Executed by whole groups.
     auto store_bag = [&](int bag, int L) {
         const float mm = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
         const float bm = bias_acc * mm;
         // (computed here, once per bag, rather than kept in registers across the row loop)
         const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
-        char* seg = p.dests ? dest_segment(p, b0 + bag, m.col, esz)
-                            : static_cast<char*>(p.output) + ((b0 + bag) * p.out_stride + m.col) * esz;
+        char* seg = p.dests ? dest_segment(p, b0 + bag, m.col, esz) : out0 + static_cast<int64_t>(bag) * (p.out_stride * esz);
         const bool vec = (reinterpret_cast<uintptr_t>(seg) & 15) == 0;
         bool stored = false;
         if constexpr (FOLD) {
@@ -1151,7 +689,7 @@ __device__ __noinline__ void pool_run_stream(const LookupParams& p, const TableM
     // without reading for a row that is not to be added.
     auto request = [&](uint32_t st, int32_t idx) {
         const bool ok = act && idx >= 0;   // the lanes past the row's last unit zero-fill their slots as well
-        const uint8_t* src = ok ? lane_base + static_cast<uint64_t>(static_cast<uint32_t>(idx)) * stride : zero_base;
+        const uint8_t* src = lane_base + static_cast<uint64_t>(static_cast<uint32_t>(max(idx, 0))) * stride;
         const int sz = ok ? CH : 0;
         if constexpr (CH == 8) {
             cp_async8(my_main + st, src, sz);
@@ -1166,7 +704,7 @@ __device__ __noinline__ void pool_run_stream(const LookupParams& p, const TableM
             }
         }
         if constexpr (kHdr) {
-            if (head_lane) cp_async4(my_tail + st, src + tail_off, ok ? 4 : 0);   // (zero_base + tail_off is still inside the zeros)
+            if (head_lane) cp_async4(my_tail + st, src + tail_off, ok ? 4 : 0);
         }
         cp_async_commit();
     };
@@ -1341,61 +879,443 @@ __device__ __forceinline__ void pool_run_stream_by_type(const LookupParams& p, c
 }
 
 
-// A run of bags of one table through the general per-bag code.
-template <typename IdxT, bool STAGING>
-__device__ __forceinline__ void pool_run_general(const LookupParams& p, const TableMeta& m, int64_t i0, int64_t i1, int64_t b,
-                                                 int lane, uint32_t wsm)
+// ---- bags summed in steps of eight rows -----------------------------------------------------------------
+//
+// A warp takes its run's bags in order, a bag in steps of up to eight rows.  Lane 8 j + g owns unit g (and g + 8) of rows
+// j and j + 4 of the step, so a unit is summed by four lanes, each over its quarter of the bag's rows, and what is left
+// of a bag at its end is one exchange through shared memory: every lane takes one quad of elements from the four
+// that have summed it and stores it, 32 lanes one contiguous piece.  All of that is warp-uniform and runs once per bag, where
+// pool_run_stream runs its end of a bag once per bag AND lane group.  No row of another bag shares a step, so
+// nothing is masked: a step's missing rows are zero-filled.
+//
+// What bounds the pooled lookup is the instructions issued per row, so the arithmetic is cut as well.  A code is used where
+// it lies: masked out of its word and read as fp32 it is a subnormal (q * 2^8 * 2^-149 for the second byte), which is
+// exact, and so is its product with the row's scale times 2^111; packed fp32 FMAs (two elements each) add the
+// products with one rounding, as before.  What the place of a code multiplies is undone when the bag is stored.  One mask
+// and half an FMA per code instead of a permute and an FMA, one mask instead of three instructions for an INT4 code.
+// With per-sample weights scale * weight may have any magnitude, so the codes are made ordinary numbers first (2^23 + q in
+// one masking instruction, less 2^23 in half a packed addition).
+//
+// Row fetch.  Rows travel through a ring of NS stages in the warp's shared memory with asynchronous copies through L1, each
+// lane copying and reading back only its own bytes.  CB bytes per lane and row: 4, 8, 16 or 32, so that narrow rows keep
+// all lanes busy and one pass covers up to 256 bytes (INT4: 128); wider rows take several passes over the run, each
+// over its own columns.  Any D that is a multiple of 4 will do: a row's last unit may reach into the row's padding,
+// whose sums are not stored.
+
+// Two packed fp32 numbers, and c += a * b and a + b on them.
+__device__ __forceinline__ unsigned long long pack2(uint32_t lo, uint32_t hi)
 {
-    const IdxT* offsets = static_cast<const IdxT*>(p.offsets);
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+    return v;
+}
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ void sts16u(uint32_t a, unsigned long long x, unsigned long long y)
+{
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
+}
+
+// Asynchronous 4-byte copy by the lanes that `on` selects, predicated instead of branched around.
+__device__ __forceinline__ void cp_async4_if(bool on, uint32_t dst, const void* src, int bytes)
+{
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %3, 0; @p cp.async.ca.shared.global [%0], [%1], 4, %2; }" ::"r"(dst), "l"(src), "r"(bytes),
+                 "r"(static_cast<int>(on))
+                 : "memory");
+}
+
+constexpr int kIndexRing = 128;                        // rows whose numbers (and weights) are at hand: a power of two above what is in flight
+
+template <int TY, int CB, bool WEIGHTED>
+__device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane, uint32_t wsm)
+{
+    static_assert(CB == 4 || CB == 8 || CB == 16 || (CB == 32 && TY != TBE_B200_INT4), "at most 32 elements per lane and pass");
+    constexpr bool k8 = (TY == TBE_B200_INT8), k4 = (TY == TBE_B200_INT4), k16 = (TY == TBE_B200_FP16), kF8 = (TY == TBE_B200_FP8),
+                   k32 = (TY == TBE_B200_FP32);
+    constexpr bool kHdr = k8 || k4;
+    static_assert((!k16 || CB >= 8) && (!k32 || CB >= 16), "four elements at least");
+    constexpr int EPW = k4 ? 8 : k16 ? 2 : k32 ? 1 : 4;   // elements of a 32-bit word of the row
+    constexpr int HS = kHdr ? EPW : 0;                    // element slots of the first unit that the header takes
+    constexpr int NCH = (CB == 32) ? 2 : 1;               // units per lane and pass
+    constexpr int CHB = CB / NCH;                         // bytes of a unit: one asynchronous copy
+    constexpr int WPU = CHB / 4;                          // 32-bit words of a unit
+    constexpr int NW = CB / 4;                            // words per lane and row
+    constexpr int NQ = NW * EPW / 4;                      // quads: four elements each
+    constexpr int EPU = WPU * EPW;                        // elements of a unit
+    constexpr int HALF = kWarp * CB;                      // four rows of a stage
+    constexpr int STAGE = 2 * HALF + 32;                  // eight rows and their side words
+    constexpr int XQ = NQ < 4 ? NQ : 4;                   // quads exchanged at a time
+    constexpr int XROW = 32 + 8 / XQ;                     // (so that eight lanes' reads fall on different banks)
+    constexpr int XCHG = XQ * XROW * 16;
+    constexpr int RING = kStreamSmemBytes - kRelBytes - 2 * kIndexRing * 4 - XCHG;
+    constexpr int NS = RING / STAGE < 6 ? RING / STAGE : 6;   // stages: steps in flight
+    static_assert(NS >= 2 && NS * 8 + 2 * kWarp + 8 <= kIndexRing, "the rings do not fit");
+    const int j = lane >> 3, g = lane & 7;             // row of the step, unit: a copy instruction covers whole pieces of four rows
+    const int D = m.D;
+    const uint32_t stride = static_cast<uint32_t>(m.stride);
+    const int payload = k32 ? 4 * D : k16 ? 2 * D : k4 ? D / 2 : D;     // bytes
+    // A row that is a whole number of units without its header: the header's place in the first unit takes the row's last
+    // four bytes (the side word), so that no unit is spent on them.
+    const bool wrap = kHdr && payload % CHB == 0;
+    const int units = wrap ? payload / CHB : (payload + (kHdr ? 4 : 0) + CHB - 1) / CHB;
+    const bool idx64 = p.idx64 != 0;
+    const int isz = idx64 ? 8 : 4;
+    const uint32_t sm_rel = wsm, sm_idx = wsm + kRelBytes, sm_w = sm_idx + kIndexRing * 4, sm_x = sm_w + kIndexRing * 4, ring = sm_x + XCHG;
+
+    int64_t off = 0;
+    if (lane <= nb) {
+        const char* op = static_cast<const char*>(p.offsets) + (i0 + lane) * isz;
+        off = idx64 ? __ldg(reinterpret_cast<const int64_t*>(op)) : static_cast<int64_t>(__ldg(reinterpret_cast<const int32_t*>(op)));
+    }
+    int64_t R0 = __shfl_sync(kFull, off, 0);
+    int64_t R1 = __shfl_sync(kFull, off, nb);
+    if (R0 < 0 || R1 < R0 || R1 > p.num_indices || R1 - R0 > 0x7fffff00ll) {
+        // Offsets that do not describe positions of `indices`: nothing is read through them; the run's bags are
+        // written as empty ones (zeros), so that the output is defined, and the condition is reported.
+        if (p.error_flag && lane == 0) atomicOr(p.error_flag, 8);
+        off = R0 = R1 = 0;
+    }
+    const int n = static_cast<int>(R1 - R0);
+    int rel = static_cast<int>(min(max(off - R0, static_cast<int64_t>(0)), static_cast<int64_t>(n)));
+    if (lane > nb) rel = n;
+    // (offsets that run backwards inside the run count as the largest before them, so that the walk below only moves on)
+#pragma unroll
+    for (int d = 1; d < kWarp; d <<= 1) {
+        const int before = __shfl_up_sync(kFull, rel, d);
+        if (lane >= d) rel = max(rel, before);
+    }
+    __syncwarp();                                      // the previous run's reads of this memory are over
+    sts4(sm_rel + 4 * lane, rel);
+    const int next_rel = __shfl_down_sync(kFull, rel, 1);
+    const int total_steps = static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(lane < nb ? (next_rel - rel + 7) >> 3 : 0)));
+    __syncwarp();
+
+    const char* ipb = static_cast<const char*>(p.indices) + (R0 + lane) * isz;
+    const float* wpb = WEIGHTED ? p.pw + R0 + lane : nullptr;
+    const uint64_t rows_avail = static_cast<uint64_t>(m.avail) / stride;
+    const uint64_t max_rows = rows_avail < 0x80000000ull ? rows_avail : 0x80000000ull;
+    const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
+    constexpr float kScaleUp = 0x1p111f, kUnit = 0x1p-38f;              // unweighted codes: 2^-149 * 2^111
+    constexpr float kFp8W = 0x1p60f;                                    // weighted FP8: so much of fp8_mult is in the weights
+    const float mul_base = kHdr ? (WEIGHTED ? 1.0f : 1.0f / kUnit) : kF8 ? (WEIGHTED ? p.fp8_mult / kFp8W : p.fp8_mult) : 1.0f;
+
+    for (int u0 = 0; u0 < units; u0 += 8 * NCH) {
+        const bool first_pass = (u0 == 0);
+        // The side word (lanes 0, 8, 16 and 24, one per row): the row's tail in the first pass of a wrapped row, the header in later ones.
+        const bool side_lane = kHdr && g == 0 && (wrap || !first_pass);
+        const uint8_t* lane_base = m.table + (u0 + g) * CHB;
+        const uint8_t* side_base = m.table + (first_pass ? payload : 0);
+        const int size0 = u0 + g < units ? CHB : 0, size1 = u0 + g + 8 < units ? CHB : 0;
+
+        unsigned long long acc[2 * NQ];                // pairs of elements; 0 is (0.0f, 0.0f)
+#pragma unroll
+        for (int i = 0; i < 2 * NQ; ++i) acc[i] = 0ull;
+        float bias_acc = 0.0f;
+
+        // Indices are loaded 32 at a time, two chunks ahead, kept as loaded until their chunk's turn (anything computed from
+        // them earlier would wait for the load), then narrowed and put into the ring.  -1 = nothing to add; a row outside
+        // [-1, 2^31) or past the end of the table is reported and skipped.
+        uint2 raw_a, raw_b;
+        float w_a = 0.0f, w_b = 0.0f;
+        auto load_raw = [&](int c, uint2& raw, float& w) {
+            raw = make_uint2(0xffffffffu, 0xffffffffu);
+            if (c * kWarp + lane < n) {
+                const char* ip = ipb + static_cast<int64_t>(c) * (kWarp * isz);
+                if (idx64) raw = ld_once_2x32(ip);
+                else raw.x = static_cast<uint32_t>(ld_once32(ip));
+                if constexpr (WEIGHTED) w = ld_once_f32(wpb + c * kWarp);
+            }
+        };
+        auto put_chunk = [&](int c, uint2 words, float w) {
+            const int64_t raw = idx64 ? static_cast<int64_t>((static_cast<uint64_t>(words.y) << 32) | words.x)
+                                      : static_cast<int64_t>(static_cast<int32_t>(words.x));
+            int32_t idx = static_cast<int32_t>(raw);
+            if (static_cast<uint64_t>(raw) >= max_rows) {          // -1 and every other negative number included
+                if (raw != -1 && p.error_flag) atomicOr(p.error_flag, (raw < 0 || raw > 0x7fffffffll) ? 1 : 4);
+                idx = -1;
+            }
+            const uint32_t at = static_cast<uint32_t>((c * kWarp + lane) & (kIndexRing - 1)) * 4u;
+            sts4(sm_idx + at, idx);
+            if constexpr (WEIGHTED) sts4(sm_w + at, __float_as_int(idx >= 0 ? w : 0.0f));
+            __syncwarp();
+        };
+
+        const uint32_t my_main = ring + static_cast<uint32_t>(lane) * CHB;
+        const uint32_t my_side = ring + 2 * HALF + static_cast<uint32_t>(j) * 4u;
+        // Requests this lane's bytes of row `idx` into half h of the stage; a row that is not to be added is zero-filled.
+        auto request_row = [&](uint32_t st, int h, int32_t idx) {
+            const uint64_t at = static_cast<uint64_t>(static_cast<uint32_t>(max(idx, 0))) * stride;
+            const uint32_t dst = my_main + st + h * HALF;
+            // (lanes past the row's last unit zero-fill as well: no branch)
+            if constexpr (CHB == 4) cp_async4(dst, lane_base + at, idx >= 0 ? size0 : 0);
+            else if constexpr (CHB == 8) cp_async8(dst, lane_base + at, idx >= 0 ? size0 : 0);
+            else cp_async16_ca(dst, lane_base + at, idx >= 0 ? size0 : 0);
+            if constexpr (NCH == 2) cp_async16_ca(dst + kWarp * 16, lane_base + at + 128, idx >= 0 ? size1 : 0);
+            if constexpr (kHdr) cp_async4_if(side_lane, my_side + st + h * 16, side_base + at, idx >= 0 ? 4 : 0);
+        };
+
+        // Adds this lane's words of one row.  `hdr` is the row's header, w its weight.
+        auto add_row = [&](const uint32_t (&r)[NW], uint32_t hdr, float w) {
+            if constexpr (kHdr) {
+                const float sc = half_bits_to_float(hdr & 0xffffu), bi = half_bits_to_float(hdr >> 16);
+                bias_acc = WEIGHTED ? fmaf(bi, w, bias_acc) : bias_acc + bi;
+                const uint32_t s = __float_as_uint(WEIGHTED ? sc * w : sc * kScaleUp);
+                const unsigned long long ss = pack2(s, s);
+                // 2^23 + q when the codes are to be ordinary numbers
+                constexpr uint32_t kM = WEIGHTED ? 0x4B000000u : 0u;
+                const unsigned long long minus = pack2(0xCB000000u, 0xCB000000u);
+                auto two = [&](uint32_t a, uint32_t b) { return WEIGHTED ? add2(pack2(a, b), minus) : pack2(a, b); };
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    const uint32_t x = r[i];
+                    if constexpr (k8) {
+                        fma2(acc[2 * i], two((x & 0xFFu) | kM, (x & 0xFF00u) | kM), ss);
+                        fma2(acc[2 * i + 1], two((x & 0xFF0000u) >> (WEIGHTED ? 8 : 0) | kM, (x >> 24) | kM), ss);
+                    } else {
+                        const uint32_t y = x >> 24;
+                        fma2(acc[4 * i], two((x & 0xFu) | kM, (x & 0xF0u) | kM), ss);
+                        fma2(acc[4 * i + 1], two((x & 0xF00u) | kM, (x & 0xF000u) | kM), ss);
+                        fma2(acc[4 * i + 2], two((x & 0xF0000u) | kM, (WEIGHTED ? (x >> 20) & 0xFu : x & 0xF00000u) | kM), ss);
+                        fma2(acc[4 * i + 3], two((y & 0xFu) | kM, (y & 0xF0u) | kM), ss);
+                    }
+                }
+            } else if constexpr (kF8) {
+                // byte -> bf16, two at a time: sign to the top, the rest to exponent and mantissa; a bf16 is the upper half of an fp32
+                const uint32_t sh = p.fp8_shift - 16;
+                const uint32_t s = __float_as_uint(WEIGHTED ? w * kFp8W : 1.0f);
+                const unsigned long long ss = pack2(s, s);
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    const uint32_t x = r[i], y = x >> 8;
+                    const uint32_t even = ((x & 0x007F007Fu) << sh) | ((x & 0x00800080u) << 8), odd = ((y & 0x007F007Fu) << sh) | ((y & 0x00800080u) << 8);
+                    fma2(acc[2 * i], pack2(even << 16, odd << 16), ss);
+                    fma2(acc[2 * i + 1], pack2(even & 0xffff0000u, odd & 0xffff0000u), ss);
+                }
+            } else if constexpr (k32) {
+                const uint32_t s = __float_as_uint(w);
+                const unsigned long long ss = pack2(s, s);
+#pragma unroll
+                for (int i = 0; i < NW / 2; ++i) {
+                    if constexpr (WEIGHTED) fma2(acc[i], pack2(r[2 * i], r[2 * i + 1]), ss);
+                    else acc[i] = add2(acc[i], pack2(r[2 * i], r[2 * i + 1]));
+                }
+            } else {
+                const uint32_t s = __float_as_uint(w);
+                const unsigned long long ss = pack2(s, s);
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[i]));
+                    const unsigned long long v = pack2(__float_as_uint(f.x), __float_as_uint(f.y));
+                    if constexpr (WEIGHTED) fma2(acc[i], v, ss);
+                    else acc[i] = add2(acc[i], v);
+                }
+            }
+        };
+
+        // Adds the (up to) eight rows in stage `st`, rows pos .. min(pos + 8, end) - 1 of the run.
+        auto consume = [&](uint32_t st, int pos, int end) {
+            uint32_t r[2][NW];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t src = my_main + st + h * HALF;
+                if constexpr (CHB == 4) {
+                    r[h][0] = lds4(src);
+                } else if constexpr (CHB == 8) {
+                    const uint2 v = lds8(src);
+                    r[h][0] = v.x;
+                    r[h][1] = v.y;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) {
+                        const uint4 v = lds16(src + c * (kWarp * 16));
+                        r[h][4 * c + 0] = v.x;
+                        r[h][4 * c + 1] = v.y;
+                        r[h][4 * c + 2] = v.z;
+                        r[h][4 * c + 3] = v.w;
+                    }
+                }
+            }
+            uint32_t hdr[2] = {0u, 0u};
+            if constexpr (kHdr) {
+                uint32_t word[2] = {r[0][0], r[1][0]};
+                // read by every lane (no branch); the tails take the headers' places in a wrapped row's first pass
+                const uint32_t s0 = lds4(my_side + st), s1 = lds4(my_side + st + 16);
+                if (side_lane) {
+                    word[0] = first_pass ? word[0] : s0;
+                    word[1] = first_pass ? word[1] : s1;
+                    r[0][0] = first_pass ? s0 : r[0][0];
+                    r[1][0] = first_pass ? s1 : r[1][0];
+                }
+                hdr[0] = __shfl_sync(kFull, word[0], lane & 24);   // from the lane of unit 0; zero for a row that was not copied
+                hdr[1] = __shfl_sync(kFull, word[1], lane & 24);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float w = 1.0f;
+                if constexpr (WEIGHTED) {
+                    const int at = pos + 4 * h + j;
+                    w = __int_as_float(lds4i(sm_w + static_cast<uint32_t>(at & (kIndexRing - 1)) * 4u));
+                    w = at < end ? w : 0.0f;                       // (what is found past the bag's end belongs to another bag)
+                }
+                add_row(r[h], hdr[h], w);
+            }
+        };
+
+        // Stores bag `bag` of L rows, and clears the sums.
+        auto finish_bag = [&](int bag, int L) {
+            bias_acc += __shfl_xor_sync(kFull, bias_acc, 8);
+            bias_acc += __shfl_xor_sync(kFull, bias_acc, 16);
+            const float mm = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
+            const float mul = mul_base * mm, bm = bias_acc * mm;
+            char* seg = p.dests ? dest_segment(p, b0 + bag, m.col, esz) : static_cast<char*>(p.output) + ((b0 + bag) * p.out_stride + m.col) * esz;
+            const bool vec = (reinterpret_cast<uintptr_t>(seg) & (4 * esz - 1)) == 0;     // element positions are multiples of 4
+#pragma unroll
+            for (int x0 = 0; x0 < NQ; x0 += XQ) {
+                __syncwarp();                          // the previous exchange has been read
+#pragma unroll
+                for (int i = 0; i < XQ; ++i) sts16u(sm_x + static_cast<uint32_t>(i * XROW + lane) * 16u, acc[2 * (x0 + i)], acc[2 * (x0 + i) + 1]);
+                __syncwarp();
+                const int xu = lane / XQ, q = x0 + lane % XQ;     // the unit (of eight) and the quad this lane finishes
+                if (xu < 8) {
+                    const uint32_t from = sm_x + static_cast<uint32_t>((lane % XQ) * XROW + xu) * 16u;
+                    const float4 a = lds16f(from), b = lds16f(from + 128), c = lds16f(from + 256), d = lds16f(from + 384);
+                    // what a code's place in its word multiplied
+                    float m0 = mul, m1 = mul, m2 = mul, m3 = mul;
+                    if constexpr (k8) {
+                        m1 = mul * 0x1p-8f;
+                        m2 = WEIGHTED ? m1 : mul * 0x1p-16f;
+                    } else if constexpr (k4) {
+                        const bool upper = q & 1;      // nibbles 4 .. 7 of the word
+                        m0 = upper ? mul * 0x1p-16f : mul;
+                        m1 = upper ? (WEIGHTED ? mul : mul * 0x1p-20f) : mul * 0x1p-4f;
+                        m2 = upper ? mul : mul * 0x1p-8f;
+                        m3 = upper ? mul * 0x1p-4f : mul * 0x1p-12f;
+                    }
+                    const float v[4] = {fmaf((a.x + b.x) + (c.x + d.x), m0, bm), fmaf((a.y + b.y) + (c.y + d.y), m1, bm),
+                                        fmaf((a.z + b.z) + (c.z + d.z), m2, bm), fmaf((a.w + b.w) + (c.w + d.w), m3, bm)};
+                    constexpr int QPU = EPU / 4;       // quads of a unit
+                    const int unit = u0 + xu + 8 * (q / QPU);
+                    int e0 = EPU * unit - HS + 4 * (q % QPU);
+                    if (kHdr && unit == 0 && q % QPU < HS / 4) e0 = wrap ? D - HS + 4 * q : -1;
+                    if (unit < units && e0 >= 0 && e0 < D) store_out<4>(seg, e0, v, p.out_ty, vec);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * NQ; ++i) acc[i] = 0ull;
+            bias_acc = 0.0f;
+        };
+
+        load_raw(0, raw_a, w_a);
+        load_raw(1, raw_b, w_b);
+        int chunks = 0;                                // chunks in the index ring
+        // the walk of the requests, and that of the sums NS steps behind it: bag, next row, end of the bag
+        int r_bag = 0, r_pos = 0, r_end = lds4i(sm_rel + 4);
+        int c_bag = 0, c_pos = 0, c_end = r_end;
+        uint32_t st = 0;
+#pragma unroll 1
+        for (int q = 0; q < total_steps + NS; ++q) {
+            if (q >= NS) {
+                while (c_pos == c_end) {               // empty bags
+                    finish_bag(c_bag, 0);
+                    c_end = lds4i(sm_rel + 4 * (++c_bag + 1));
+                }
+                cp_async_wait<NS - 1>();
+                consume(st, c_pos, c_end);
+                c_pos = min(c_pos + 8, c_end);
+                if (c_pos == c_end) {
+                    finish_bag(c_bag, c_end - lds4i(sm_rel + 4 * c_bag));
+                    ++c_bag;
+                    c_end = c_bag < nb ? lds4i(sm_rel + 4 * (c_bag + 1)) : -1;
+                }
+            }
+            if (q < total_steps) {
+                while (r_pos == r_end) r_end = lds4i(sm_rel + 4 * (++r_bag + 1));
+                while (chunks * kWarp < min(r_pos + 8, n)) {
+                    put_chunk(chunks, raw_a, w_a);
+                    raw_a = raw_b;
+                    w_a = w_b;
+                    ++chunks;
+                    load_raw(chunks + 1, raw_b, w_b);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int at = r_pos + 4 * h + j;
+                    int32_t idx = lds4i(sm_idx + static_cast<uint32_t>(at & (kIndexRing - 1)) * 4u);
+                    idx = at < r_end ? idx : -1;
+                    request_row(st, h, idx);
+                }
+                r_pos = min(r_pos + 8, r_end);
+            }
+            cp_async_commit();
+            st = (st + STAGE == NS * STAGE) ? 0u : st + STAGE;
+        }
+        cp_async_wait<0>();                            // nothing of this pass is still on its way when the ring is handed on
+        while (c_bag < nb) finish_bag(c_bag++, 0);     // empty bags at the end
+        __syncwarp();
+    }
+}
+
+template <int TY, bool WEIGHTED>
+__device__ __forceinline__ void pool_run_steps_by_width(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
+                                                        uint32_t wsm)
+{
+    // The narrowest unit with which eight lanes cover the row, so that narrow rows keep all of them busy.
+    constexpr int kHead = (TY == TBE_B200_INT8 || TY == TBE_B200_INT4) ? 4 : 0;
+    const int bytes = TY == TBE_B200_FP32 ? 4 * m.D : TY == TBE_B200_FP16 ? 2 * m.D : TY == TBE_B200_INT4 ? m.D / 2 : m.D;
+    auto covers = [&](int unit) { return bytes <= 8 * unit && (bytes % unit == 0 || bytes + kHead <= 8 * unit); };
+    if constexpr (kHead != 0 || TY == TBE_B200_FP8) {
+        if (covers(4)) { pool_run_steps<TY, 4, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return; }
+    }
+    if constexpr (TY != TBE_B200_FP32) {
+        if (covers(8)) { pool_run_steps<TY, 8, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return; }
+    }
+    if constexpr (TY == TBE_B200_INT4) {
+        pool_run_steps<TY, 16, WEIGHTED>(p, m, i0, nb, b0, lane, wsm);
+    } else {
+        if (covers(16)) pool_run_steps<TY, 16, WEIGHTED>(p, m, i0, nb, b0, lane, wsm);
+        else pool_run_steps<TY, 32, WEIGHTED>(p, m, i0, nb, b0, lane, wsm);
+    }
+}
+
+template <bool WEIGHTED>
+__device__ __forceinline__ void pool_run_steps_by_type(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
+                                                       uint32_t wsm)
+{
+    switch (m.ty) {
+        case TBE_B200_INT8: pool_run_steps_by_width<TBE_B200_INT8, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
+        case TBE_B200_INT4: pool_run_steps_by_width<TBE_B200_INT4, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
+        case TBE_B200_FP8: pool_run_steps_by_width<TBE_B200_FP8, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
+        case TBE_B200_FP16: pool_run_steps_by_width<TBE_B200_FP16, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
+        default: pool_run_steps_by_width<TBE_B200_FP32, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
+    }
+}
+
+// A run of bags of one table through the byte-wise code.
+template <typename IdxT>
+__device__ __noinline__ void pool_run_bytewise(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b, int lane)
+{
+    const IdxT* offsets = static_cast<const IdxT*>(p.offsets) + i0;
     const IdxT* indices = static_cast<const IdxT*>(p.indices);
     const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
-    int64_t start = static_cast<int64_t>(offsets[i0]);
-    for (int64_t i = i0; i < i1; ++i, ++b) {
+    int64_t start = static_cast<int64_t>(offsets[0]);
+    for (int i = 0; i < nb; ++i, ++b) {
         const int64_t end = static_cast<int64_t>(offsets[i + 1]);
         const int L = static_cast<int>(end - start);
-        BagInfo bag;
-        bag.table = m.table;
-        bag.avail = m.avail;
-        bag.stride = m.stride;
-        bag.start = start;
-        bag.L = L;
-        bag.D = m.D;
-        bag.mean_mul = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
-        char* dst;
-        int64_t brow = b;
-        if (p.dests) {
-            const int64_t which = b / p.rows_per_dest;
-            brow = b - which * p.rows_per_dest;
-            dst = static_cast<char*>(p.dests[which]);
-        } else {
-            dst = static_cast<char*>(p.output);
-        }
-        bag.seg = dst + (brow * p.out_stride + m.col) * esz;
-        bag.seg_aligned = (reinterpret_cast<uintptr_t>(bag.seg) & 15) == 0;
-        bool done = false;
-        if (STAGING && m.rows_aligned && (m.D & 3) == 0 && L >= 0 && start >= 0 && end <= p.num_indices) {
-            const BagHead head = load_batch<IdxT>(indices + start, p.pw ? p.pw + start : nullptr, min(L, kWarp), lane, p.error_flag,
-                                                  m.stride, m.avail);
-            done = true;
-            switch (m.ty) {
-                case TBE_B200_INT8: pool_bag_by_width<TBE_B200_INT8, IdxT>(p, bag, head, lane, wsm); break;
-                case TBE_B200_INT4: pool_bag_by_width<TBE_B200_INT4, IdxT>(p, bag, head, lane, wsm); break;
-                case TBE_B200_FP8: pool_bag_by_width<TBE_B200_FP8, IdxT>(p, bag, head, lane, wsm); break;
-                case TBE_B200_FP16:
-                    if ((m.D & 7) == 0) pool_bag_by_width<TBE_B200_FP16, IdxT>(p, bag, head, lane, wsm);
-                    else done = false;
-                    break;
-                case TBE_B200_FP32: pool_bag_by_width<TBE_B200_FP32, IdxT>(p, bag, head, lane, wsm); break;
-                default: done = false; break;
-            }
-        }
-        if (!done) {
-            // positions outside `indices` are not read: the bag is written as if it were empty, and reported
-            const bool sane = L >= 0 && start >= 0 && end <= p.num_indices;
-            if (!sane && lane == 0 && p.error_flag) atomicOr(p.error_flag, 8);
-            pool_bag_bytewise<IdxT>(indices + start, p.pw ? p.pw + start : nullptr, p.error_flag, bag.table, bag.stride, sane ? L : 0,
-                                    m.D, bag.seg, bag.mean_mul, m.ty, p.out_ty, p.fp8_shift, p.fp8_mult, lane, m.avail);
-        }
+        const float mean_mul = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
+        char* seg = p.dests ? dest_segment(p, b, m.col, esz) : static_cast<char*>(p.output) + (b * p.out_stride + m.col) * esz;
+        // positions outside `indices` are not read: the bag is written as if it were empty, and reported
+        const bool sane = L >= 0 && start >= 0 && end <= p.num_indices;
+        if (!sane && lane == 0 && p.error_flag) atomicOr(p.error_flag, 8);
+        pool_bag_bytewise<IdxT>(indices + start, p.pw ? p.pw + start : nullptr, p.error_flag, m.table, m.stride, sane ? L : 0, m.D, seg, mean_mul,
+                                m.ty, p.out_ty, p.fp8_shift, p.fp8_mult, lane, m.avail);
         start = end;
     }
 }
@@ -1417,77 +1337,69 @@ constexpr int kWarpsPerBlock = TBE_WARPS_PER_BLOCK;
 #define TBE_STREAM_BLOCKS_PER_SM (16 / TBE_WARPS_PER_BLOCK)   // 16 resident warps per SM at up to 128 registers (32 accumulators per lane); measured best
 #endif
 constexpr int kStreamBlocksPerSM = TBE_STREAM_BLOCKS_PER_SM;
-constexpr int kWideBlocksPerSM = 32 / TBE_WARPS_PER_BLOCK;
 
 // The T*B bags (bag i = t*B + b) are cut into spans of `span` consecutive bags, one span per warp, so a
 // warp walks `offsets`, `indices` and the per-sample weights front to back.  A span is processed as runs
 // of consecutive bags of one table: the table's description is read once per run and the run is handed
-// to the code specialised for its row shape.
-// Two builds of the kernel share this outline.  WIDE = false is the one for the common shapes: every table with
-// aligned rows of D = 16 * n <= 512 elements goes through the register streams (little shared memory, so most of
-// the SM's memory is L1 for the hot rows), anything else through the byte-wise path.  WIDE = true is launched when
-// the widest table has more than 512 elements or a width that is not a multiple of 16: aligned shapes use the
-// cp.async staging of pool_bag there.
-template <typename IdxT, bool WIDE>
-__global__ void __launch_bounds__(kWarpsPerBlock* kWarp, WIDE ? kWideBlocksPerSM : kStreamBlocksPerSM)
-tbe_pooled_kernel(const __grid_constant__ LookupParams p)
+// to the code specialised for its row shape.  pool_run_stream is inlined here (in a function of its own every memory
+// instruction has its descriptor moved into uniform registers again and the arguments are read through a pointer: 206
+// instead of 177 instructions per step of eight 128-byte rows); what a run does not need is not kept across it but
+// computed anew behind it, which leaves the row loop without spills (with them the loop is slower than the function was).
+// 64 INT8 tables of 128, batch 65536: 4.05 -> 3.83 ms; INT4 of 64/128/256: 1.72 -> 1.52 ms.
+template <bool WEIGHTED>
+__global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe_pooled_kernel(const __grid_constant__ LookupParams p)
 {
-    constexpr int kSmemPerWarp = WIDE ? kWarpSmemBytes : kStreamSmemBytes;
-    extern __shared__ __align__(128) uint8_t smem[];      // kWarpsPerBlock * kSmemPerWarp bytes, given at launch
+    extern __shared__ __align__(128) uint8_t smem[];      // kWarpsPerBlock * kStreamSmemBytes bytes, given at launch
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const uint32_t wsm = smem_u32(smem) + warp * kSmemPerWarp;
-    const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + warp;
-    const int64_t span_lo = gw * p.span;
-    const int64_t span_hi = min(p.num_bags, span_lo + p.span);
-    if (span_lo >= span_hi) return;
-    // The span's first offsets are needed right after the table description: ask for their line(s) now, so the two
-    // latencies overlap.
-    if (lane < 2) {
-        const IdxT* o = static_cast<const IdxT*>(p.offsets) + (lane == 0 ? span_lo : span_hi);
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(o));
-    }
-    // The last offset has to be the number of indices (the reference kernel asserts the same:
-    // c310/op_kernel/int_nbit_split_embedding_pooling_kernel.h:149-150); here it is reported, not trapped.
-    if (gw == 0 && lane == 0 && p.error_flag) {
-        if (static_cast<int64_t>(static_cast<const IdxT*>(p.offsets)[p.num_bags]) != p.num_indices) atomicOr(p.error_flag, 8);
+    const uint32_t wsm = smem_u32(smem) + (threadIdx.x >> 5) * kStreamSmemBytes;
+    {
+        const int64_t gw = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
+        const int64_t lo = gw * p.span;
+        if (lo >= p.num_bags) return;
+        // The span's first offsets are needed right after the table description: ask for their line(s) now, so the two
+        // latencies overlap.
+        if (lane < 2) {
+            const char* o = static_cast<const char*>(p.offsets) + (lane == 0 ? lo : min(p.num_bags, lo + p.span)) * (p.idx64 ? 8 : 4);
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(o));
+        }
+        // The last offset has to be the number of indices (the reference kernel asserts the same:
+        // c310/op_kernel/int_nbit_split_embedding_pooling_kernel.h:149-150); here it is reported, not trapped.
+        if (gw == 0 && lane == 0 && p.error_flag) {
+            const int64_t last = p.idx64 ? static_cast<const int64_t*>(p.offsets)[p.num_bags]
+                                         : static_cast<int64_t>(static_cast<const int32_t*>(p.offsets)[p.num_bags]);
+            if (last != p.num_indices) atomicOr(p.error_flag, 8);
+        }
     }
 
-    int t;
-    int64_t b;
-    if (p.B32) {
-        t = static_cast<int>(static_cast<uint32_t>(span_lo) / p.B32);
-        b = static_cast<uint32_t>(span_lo) - static_cast<uint32_t>(t) * p.B32;
-    } else {
-        t = static_cast<int>(span_lo / p.B);
-        b = span_lo - static_cast<int64_t>(t) * p.B;
-    }
-    const bool weighted = p.pw != nullptr;
-
-    for (int64_t i = span_lo; i < span_hi;) {
-        const int64_t run_end = min(span_hi, i + (p.B - b));   // the bags left in table t, or in the span
+#pragma unroll 1
+    for (int done = 0; done < p.span;) {
+        uint32_t block;                                    // (read anew for every run)
+        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
+        const int64_t i = (static_cast<int64_t>(block) * kWarpsPerBlock + (threadIdx.x >> 5)) * p.span + done;
+        if (i >= p.num_bags) break;
+        int t;
+        int64_t b;
+        if (p.B32) {
+            t = static_cast<int>(static_cast<uint32_t>(i) / p.B32);
+            b = static_cast<uint32_t>(i) - static_cast<uint32_t>(t) * p.B32;
+        } else {
+            t = static_cast<int>(i / p.B);
+            b = i - static_cast<int64_t>(t) * p.B;
+        }
+        // the bags left in the span, in table t and at all
+        const int nb = static_cast<int>(min(min(p.span - done, p.B - b), p.num_bags - i));
         const TableMeta m = load_meta(p, t);
-        if (m.D > 0) {
-            bool done = false;
-            if constexpr (!WIDE) {
-                const bool stream = m.rows_aligned && (m.D & 15) == 0 && m.D <= 512 && m.stride < (1ll << 32) &&
-                                    (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP8 ||
-                                     m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32);
-                if (stream) {
-                    const int nb = static_cast<int>(run_end - i);   // <= span <= kMaxRunBags
-                    if (weighted) pool_run_stream_by_type<true>(p, m, i, nb, b, lane, wsm);
-                    else pool_run_stream_by_type<false>(p, m, i, nb, b, lane, wsm);
-                    done = true;
-                }
-            }
-            if (!done) pool_run_general<IdxT, WIDE>(p, m, i, run_end, b, lane, wsm);
-        }
-        b += run_end - i;
-        i = run_end;
-        if (b == p.B) {
-            b = 0;
-            ++t;
-        }
+        const bool aligned = m.D > 0 && m.rows_aligned && (m.D & 3) == 0 && m.stride < (1ll << 32) &&
+                             (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32 ||
+                              (m.ty == TBE_B200_FP8 && p.fp8_shift <= 23));
+        // Widths that give every lane of a row the same 16 elements go through the streams, which issue a third fewer instructions
+        // there (64 INT8 tables of 128: 3.83 ms against 6.0 in steps; INT4 of 64/128/256: 1.52 against 1.91 ms); all others in
+        // steps (16 tables of 20 to 1024 elements of four types: 194 us; 342 us one bag at a time or byte by byte).
+        if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
+        else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
+        else if (m.D > 0 && p.idx64) pool_run_bytewise<int64_t>(p, m, i, nb, b, lane);
+        else if (m.D > 0) pool_run_bytewise<int32_t>(p, m, i, nb, b, lane);
+        done += nb;
     }
 }
 
@@ -1734,7 +1646,7 @@ constexpr int kSpanLarge = TBE_SPAN_LARGE;   // bags per warp when there is plen
 template <typename Kernel>
 int resident_blocks(Kernel kernel, int variant, int fallback, int smem_bytes = 0)
 {
-    constexpr int kMaxDev = 64, kVariants = 4;
+    constexpr int kMaxDev = 64, kVariants = 2;
     static std::atomic<int> cached[kMaxDev][kVariants];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return fallback;
@@ -1794,12 +1706,11 @@ int forced_span()
     return span;
 }
 
-template <typename IdxT, bool WIDE>
+template <bool WEIGHTED>
 int launch_pooled(LookupParams p, cudaStream_t s)
 {
-    constexpr int kSmemBytes = kWarpsPerBlock * (WIDE ? kWarpSmemBytes : kStreamSmemBytes);
-    const int resident = resident_blocks(tbe_pooled_kernel<IdxT, WIDE>, (sizeof(IdxT) == 8 ? 2 : 0) + (WIDE ? 1 : 0),
-                                         WIDE ? kWideBlocksPerSM : kStreamBlocksPerSM, kSmemBytes);
+    constexpr int kSmemBytes = kWarpsPerBlock * kStreamSmemBytes;
+    const int resident = resident_blocks(tbe_pooled_kernel<WEIGHTED>, WEIGHTED ? 1 : 0, kStreamBlocksPerSM, kSmemBytes);
     // Plenty of bags: fixed spans, as many blocks as that takes; the hardware block scheduler evens out the load.
     // Otherwise the spans are sized so that the warps fill a whole number of waves of resident warps.
     const int64_t slots = static_cast<int64_t>(sm_count()) * resident * kWarpsPerBlock;
@@ -1815,7 +1726,7 @@ int launch_pooled(LookupParams p, cudaStream_t s)
     const int64_t warps = (p.num_bags + p.span - 1) / p.span;
     const int64_t blocks = (warps + kWarpsPerBlock - 1) / kWarpsPerBlock;
     if (blocks > 0x7fffffffll) return fail(TBE_B200_ERR_UNSUPPORTED, "lookup: too many bags for one launch");
-    tbe_pooled_kernel<IdxT, WIDE><<<static_cast<unsigned>(blocks), kWarpsPerBlock * kWarp, kSmemBytes, s>>>(p);
+    tbe_pooled_kernel<WEIGHTED><<<static_cast<unsigned>(blocks), kWarpsPerBlock * kWarp, kSmemBytes, s>>>(p);
     return check_launch("tbe_pooled_kernel");
 }
 
@@ -1889,8 +1800,5 @@ extern "C" int tbe_b200_int_nbit_lookup(const tbe_b200_lookup_args* a, tbe_b200_
     }
     if (p.num_bags == 0) return TBE_B200_OK;
     if (l2_policy_mode() == 2) apply_l2_window(a->dev_weights, a->dev_weights_bytes, s);
-    // The widest table decides which build of the kernel runs (max_D is the caller's, like the reference's max_*_D).
-    const bool wide = a->max_D > 512 || (a->max_D & 15) != 0;
-    if (a->index_bits == 32) return wide ? launch_pooled<int32_t, true>(p, s) : launch_pooled<int32_t, false>(p, s);
-    return wide ? launch_pooled<int64_t, true>(p, s) : launch_pooled<int64_t, false>(p, s);
+    return p.pw ? launch_pooled<true>(p, s) : launch_pooled<false>(p, s);
 }

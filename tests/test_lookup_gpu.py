@@ -337,6 +337,102 @@ def test_bags_that_straddle_lane_group_ranges(weights_ty, D, weighted):
             run(c, pooling, out_ty, f"straddle B={B}")
 
 
+# ---- bags summed in steps of eight rows: edges of the unit widths, precision, operands that are not finite -----------------
+
+def _pool_64(c, pooling):
+    """The lookup in float64 and, for every output element, the sum of the magnitudes that went into it."""
+    out, mag = np.zeros((c.B, c.total_D)), np.zeros((c.B, c.total_D))
+    for t in range(c.T):
+        E, D, ty = c.rows[t], c.dims[t], c.tys[t]
+        rb = O.row_bytes(ty, D, c.row_alignment)
+        rows = c.dev_weights[c.weights_offsets[t]:c.weights_offsets[t] + E * rb].reshape(E, rb)
+        scale, bias = np.ones((E, 1)), np.zeros((E, 1))
+        if ty in (O.INT8, O.INT4):
+            head = rows[:, :4].copy().view(np.float16).astype(np.float64)
+            scale, bias = head[:, :1], head[:, 1:]
+            codes = rows[:, 4:4 + D] if ty == O.INT8 else np.stack([rows[:, 4:4 + D // 2] & 15, rows[:, 4:4 + D // 2] >> 4], 2).reshape(E, D)
+        elif ty == O.FP16:
+            codes = rows[:, :2 * D].copy().view(np.float16)
+        else:
+            b = rows[:, :D].astype(np.int64)
+            e, m = (b >> 3) & 15, (b & 7) / 8.0
+            codes = np.where(b >> 7, -1.0, 1.0) * np.where(e > 0, (1.0 + m) * 2.0 ** (e - 7.0), m * 2.0 ** -6)
+        part = codes.astype(np.float64) * scale
+        do = slice(c.D_offsets[t], c.D_offsets[t + 1])
+        for b in range(c.B):
+            lo, hi = int(c.offsets[t * c.B + b]), int(c.offsets[t * c.B + b + 1])
+            i, w = c.indices[lo:hi].astype(np.int64), np.ones(hi - lo) if c.weights is None else c.weights[lo:hi].astype(np.float64)
+            i, w = i[i >= 0], w[i >= 0][:, None]
+            mul = 1.0 / (hi - lo) if pooling == O.MEAN and hi > lo else 1.0
+            out[b, do] = (w * (part[i] + bias[i])).sum(0) * mul
+            mag[b, do] = (np.abs(w) * (np.abs(part[i]) + np.abs(bias[i]))).sum(0) * mul
+    return out, mag
+
+
+@pytest.mark.parametrize("weights_ty,dims", [
+    (O.INT8, [4, 28, 32, 36, 60, 64]), (O.INT8, [68, 124, 128, 132]), (O.INT8, [252, 256, 260, 516]),
+    (O.INT4, [8, 56, 64, 72, 120, 128]), (O.INT4, [136, 248, 256, 264, 520]),
+    (O.FP8, [4, 32, 36, 64, 68]), (O.FP8, [128, 132, 256, 260]),
+    (O.FP16, [4, 12, 16, 32, 36]), (O.FP16, [64, 68, 128, 132, 260])])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("out_ty", [O.FP32, O.FP16, O.BF16])
+def test_row_widths_at_the_edges_of_the_units(weights_ty, dims, weighted, out_ty):
+    """Widths around the unit sizes of pool_run_steps (a row that ends in, at and just past a unit; one and several passes),
+    bags of 0 to 9 rows and a long one (step boundaries in every position), pruned rows.  Against float64: every
+    term enters with a relative error of at most 2^-22 and every addition rounds to 2^-23 of a partial sum that is
+    bounded by the sum of magnitudes, and at most one addition per row is made."""
+    rng = np.random.default_rng(seed_of(weights_ty, dims, weighted))
+    T, B = len(dims), 21
+    lens = rng.integers(0, 10, T * B)
+    lens[3] = 67
+    c = make_case(rng, [weights_ty] * T, dims, [50] * T, B, lens, np.int64 if weighted else np.int32, weighted, prune_frac=0.03)
+    for pooling in (O.SUM, O.MEAN):
+        want, mag = _pool_64(c, pooling)
+        got = gpu_lookup(c, pooling, out_ty).astype(np.float64)
+        rows = np.repeat((c.offsets[1:] - c.offsets[:-1]).reshape(T, B).T, dims, axis=1)
+        half_ulp = {O.FP32: 0.0, O.FP16: 2.0 ** -11, O.BF16: 2.0 ** -8}[out_ty]
+        bound = mag * (2.0 ** -22 + rows * 2.0 ** -23) + np.abs(want) * half_ulp * 1.01 + (2.0 ** -25 if out_ty == O.FP16 else 1e-38)
+        assert np.all(np.abs(got - want) <= bound), f"max excess {(np.abs(got - want) - bound).max()}"
+
+
+@pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4])
+@pytest.mark.parametrize("magnitude", [1e-30, 1e-12, 1.0, 1e12])
+def test_weights_of_any_magnitude(weights_ty, magnitude):
+    """Per-sample weights far from one, next to bags of ordinary ones: relative to the magnitudes that go in, the result
+    is as good as with weights around one."""
+    rng = np.random.default_rng(17)
+    c = make_case(rng, [weights_ty] * 2, [64, 264], [80, 90], 9, rng.integers(0, 40, 18), np.int64, True)
+    c.weights[: int(c.offsets[7])] *= np.float32(magnitude)
+    want, mag = _pool_64(c, O.SUM)
+    got = gpu_lookup(c, O.SUM, O.FP32).astype(np.float64)
+    assert np.all(np.abs(got - want) <= mag * 2.0 ** -17 + 1e-38)      # 40 rows: 2^-22 + 40 * 2^-23
+
+
+@pytest.mark.parametrize("weights_ty,weighted", [(O.FP16, False), (O.INT8, False), (O.INT8, True), (O.INT4, True)])
+def test_infinities_and_nans_stay_in_their_bag(weights_ty, weighted):
+    """A row with infinities or NaNs (FP16 payload; INT8 / INT4 bias) changes its own bag only."""
+    rng = np.random.default_rng(23)
+    c = make_case(rng, [weights_ty] * 2, [128, 36 if weights_ty != O.INT4 else 40], [60, 60], 16, rng.integers(1, 9, 32), np.int32, weighted)
+    c.indices[c.indices >= 50] = 1                      # rows 50 .. 53 are used by one bag each
+    clean = oracle_lookup(c, O.SUM, O.FP16)
+    hit, odd = [0, 5, 18, 31], [np.inf, -np.inf, np.nan, np.inf]
+    rb = [O.row_bytes(weights_ty, d, 16) for d in c.dims]
+    for k, (bag, value) in enumerate(zip(hit, odd)):
+        t = bag // 16
+        c.indices[int(c.offsets[bag])] = 50 + k
+        at = int(c.weights_offsets[t]) + (50 + k) * rb[t] + (2 * 7 if weights_ty == O.FP16 else 2)
+        c.dev_weights[at:at + 2] = np.frombuffer(np.float16(value).tobytes(), dtype=np.uint8)
+    got = gpu_lookup(c, O.SUM, O.FP16)
+    want = oracle_lookup(c, O.SUM, O.FP16)
+    for t in range(2):
+        cols = slice(c.D_offsets[t], c.D_offsets[t + 1])
+        touched = np.zeros(16, bool)
+        touched[[b - 16 * t for b in hit if b // 16 == t]] = True
+        assert np.allclose(got[~touched][:, cols], clean[~touched][:, cols], rtol=1e-3, atol=1e-3)
+        assert np.array_equal(np.isnan(got[touched][:, cols]), np.isnan(want[touched][:, cols]))
+        assert np.allclose(got[touched][:, cols], want[touched][:, cols], rtol=1e-3, atol=1e-3, equal_nan=True)
+
+
 @pytest.mark.parametrize("weights_ty,dims", [(O.INT8, [4, 12, 8, 40]), (O.INT4, [8, 40, 24, 136]), (O.FP16, [8, 20, 2, 40]), (O.FP8, [4, 24, 8, 100]),
                                              (O.FP32, [3, 4, 20, 8])])
 @pytest.mark.parametrize("out_ty", [O.FP32, O.FP16, O.BF16])
