@@ -3,16 +3,16 @@
 // Replaces the device side of int_nbit_split_embedding_codegen_lookup_function
 // (reference: c310/op_kernel/int_nbit_split_embedding_pooling_kernel.h:44-394 and
 // int_nbit_split_embedding_nobag_kernel.h:31-398).  The path is a gather and a
-// reduction bounded by HBM/L2 bandwidth, so there is no tensor-core work here.
+// reduction, bounded by the instructions issued per row and by HBM/L2 bandwidth.  Codes as operands of mma.sync with bags as
+// its columns measured slower than the packed FMAs: the instruction runs at one per 64 cycles and SM quarter here.
 //
 // Pooled kernel (SUM / MEAN), in three tiers chosen per table:
 //   * aligned rows of INT8 / INT4 / FP8 / FP16 / FP32 with D a multiple of 16 up to 512 (pool_run_stream): LPR lanes
 //     share a row, 16 fp32 accumulators per lane, so a warp has 32/LPR lane groups.  The rows of a warp's bags are
 //     cut into equal ranges, one per group, and every group streams its range through a small ring in shared
 //     memory: asynchronous 16-byte copies through L1 (which holds the hot head of a Zipf-distributed table), several
-//     rows per group in flight, consumed in order; bags that straddle two ranges are combined through shared memory.  Rows are dequantised
-//     with the row's fp16 scale/bias (codes -> exact fp16 by a magic constant, then fp16 x fp16 + fp32 mixed FMA)
-//     and accumulated in fp32.  INT8/INT4 rows start with a 4-byte header, which shifts the payload off the
+//     rows per group in flight, consumed in order; bags that straddle two ranges are combined through shared memory.  Codes
+//     are multiplied by the row's fp16 scale and accumulated in fp32 where they lie in their words (see kCodeScale).  INT8/INT4 rows start with a 4-byte header, which shifts the payload off the
 //     16-byte grid; the lane that reads the header chunk has 4 / 8 free slots, which take the row's last
 //     elements, so D = 16*LPR rows keep every lane busy with exactly 16 elements;
 //   * aligned rows of the same types and any other D that is a multiple of 4 (pool_run_steps): a warp sums its bags one after
@@ -349,70 +349,75 @@ __device__ __forceinline__ int32_t lds4i(uint32_t a)
     return v;
 }
 
-// The header of an INT8 / INT4 row (fp16 scale, fp16 bias; zero for a row that is not to be added): adds the bias
-// (and, in the folded form, the scale) to the bag's running sums and returns the scale's fp16 bits; `ws` is
-// scale * w for the weighted form.
-template <bool WEIGHTED, bool FOLD>
-__device__ __forceinline__ unsigned short accum_header(uint32_t hdr, float w, float& ws, float& bias_acc, float& scale_acc)
+// Two packed fp32 numbers, and a + b on them.
+__device__ __forceinline__ unsigned long long pack2(uint32_t lo, uint32_t hi)
 {
-    const unsigned short scale_h = static_cast<unsigned short>(hdr & 0xffffu);
-    ws = 0.0f;
-    if constexpr (WEIGHTED) {
-        ws = half_bits_to_float(scale_h) * w;
-        bias_acc = fmaf(half_bits_to_float(hdr >> 16), w, bias_acc);
-    } else {
-        bias_acc += half_bits_to_float(hdr >> 16);
-        if constexpr (FOLD) scale_acc += half_bits_to_float(scale_h);
-    }
-    return scale_h;
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+    return v;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+// c0 += a0 * b and c1 += a1 * b in one instruction.
+__device__ __forceinline__ void fma2(float& c0, float& c1, unsigned long long a, float b)
+{
+    asm("{ .reg .b64 c, d; mov.b64 c, {%0, %1}; mov.b64 d, {%3, %3}; fma.rn.f32x2 c, %2, d, c; mov.b64 {%0, %1}, c; }"
+        : "+f"(c0), "+f"(c1)
+        : "l"(a), "f"(b));
 }
 
-// Adds NW 32-bit words of INT8 (4 per word) or INT4 (8 per word) codes, times the row scale, to consecutive slots
-// of `acc` (a compile-time position inside the lane's accumulators).
-template <int TY, bool WEIGHTED, bool FOLD, int NW>
-__device__ __forceinline__ void accum_codes(const uint32_t (&words)[NW], unsigned short scale_h, float ws, float* acc)
+// (a0 * b0 + c, a1 * b1 + c) in one instruction.
+__device__ __forceinline__ float2 fma2_value(float a0, float a1, float b0, float b1, float c)
 {
-    if constexpr (TY == TBE_B200_INT8 && FOLD) {
-        // One byte permute per code builds the register the mixed FMA wants: its two fp16 operands side by side,
-        // (1024 + q) below (bytes q, 0x64) and the row scale above.  With the operands in two registers the compiler
-        // spends a move per FMA to bring them together (measured: 16 moves for 16 FMAs, none in this form).
-        const uint32_t y = (static_cast<uint32_t>(scale_h) << 16) | 0x6400u;
+    float2 v;
+    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %6}; fma.rn.f32x2 x, x, y, z; mov.b64 {%0, %1}, x; }"
+        : "=f"(v.x), "=f"(v.y)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c));
+    return v;
+}
+
+// Codes as fp32 numbers.  A code is used where it lies: masked out of its word and read as fp32 it is a subnormal
+// (q * 2^8 * 2^-149 for the second byte), which is exact, and so is its product with the row's scale times kCodeScale; one
+// packed FMA adds two of them with one rounding each, as a mixed FMA per code did, and what the place of a code
+// multiplied is undone when the bag is stored (code_unit).  With per-sample weights scale * weight may have any magnitude, so
+// the codes are made ordinary numbers first: 2^23 + q in the masking instruction, less 2^23 in half a packed addition.
+// A step of eight 128-byte rows takes 162 instructions instead of 177 with a byte permute and a mixed FMA per code: 64 INT8
+// tables of 128, batch 65536: 3.83 -> 3.74 ms; INT4 of 64/128/256: 1.52 -> 1.30 ms.
+constexpr float kCodeScale = 0x1p111f;
+template <int TY, bool WEIGHTED>
+__device__ constexpr float code_unit(int slot)
+{
+    const float base = WEIGHTED ? 1.0f : 0x1p38f;      // 1 / (2^-149 * kCodeScale)
+    if (TY == TBE_B200_INT8) return base * (slot % 4 == 1 ? 0x1p-8f : slot % 4 == 2 ? (WEIGHTED ? 0x1p-8f : 0x1p-16f) : 1.0f);
+    if (TY == TBE_B200_INT4)
+        return base * (slot % 8 == 1 || slot % 8 == 7 ? 0x1p-4f : slot % 8 == 2 ? 0x1p-8f : slot % 8 == 3 ? 0x1p-12f : slot % 8 == 4 ? 0x1p-16f
+                       : slot % 8 == 5 && !WEIGHTED ? 0x1p-20f : 1.0f);
+    return 1.0f;
+}
+
+// Adds NW 32-bit words of INT8 (4 per word) or INT4 (8 per word) codes, times `s`, to consecutive slots of `acc`.
+template <int TY, bool WEIGHTED, int NW>
+__device__ __forceinline__ void accum_codes(const uint32_t (&words)[NW], float s, float* acc)
+{
+    constexpr uint32_t kM = WEIGHTED ? 0x4B000000u : 0u;
+    const unsigned long long minus = pack2(0xCB000000u, 0xCB000000u);
+    auto two = [&](uint32_t a, uint32_t b) { return WEIGHTED ? add2(pack2(a | kM, b | kM), minus) : pack2(a, b); };
 #pragma unroll
-        for (int i = 0; i < NW; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t x = __byte_perm(words[i], y, 0x7650u | j);
-                asm("{ .reg .b16 l, h; mov.b32 {l, h}, %1; fma.rn.f32.f16 %0, l, h, %0; }" : "+f"(acc[4 * i + j]) : "r"(x));
-            }
-        }
-    } else if constexpr (TY == TBE_B200_INT8) {
-#pragma unroll
-        for (int i = 0; i < NW; ++i) {
-            const uint32_t c = words[i];
-            // bytes 0 and 2, then bytes 1 and 3, placed in the mantissas of half2(1024, 1024)
-            uint32_t even = (c & 0x00FF00FFu) | 0x64006400u;
-            uint32_t odd = __byte_perm(c, 0x64646464u, 0x4341);
-            if constexpr (!FOLD) {
-                even = codes_to_half2(even, 0x64006400u);
-                odd = codes_to_half2(odd, 0x64006400u);
-            }
-            add_pair_t<WEIGHTED>(acc[4 * i + 0], acc[4 * i + 2], even, scale_h, ws);
-            add_pair_t<WEIGHTED>(acc[4 * i + 1], acc[4 * i + 3], odd, scale_h, ws);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < NW; ++i) {
-            const uint32_t c = words[i];
-            const uint32_t y = c >> 8;
-            // nibble pairs (j, j + 4) sit 16 bits apart: 0x6400 | n = 1024 + n; 0x5400 | (n << 4) = 64 + n
-            const uint32_t p0 = codes_to_half2((c & 0x000F000Fu) | 0x64006400u, 0x64006400u);   // nibbles 0, 4
-            const uint32_t p1 = codes_to_half2((c & 0x00F000F0u) | 0x54005400u, 0x54005400u);   // nibbles 1, 5
-            const uint32_t p2 = codes_to_half2((y & 0x000F000Fu) | 0x64006400u, 0x64006400u);   // nibbles 2, 6
-            const uint32_t p3 = codes_to_half2((y & 0x00F000F0u) | 0x54005400u, 0x54005400u);   // nibbles 3, 7
-            add_pair_t<WEIGHTED>(acc[8 * i + 0], acc[8 * i + 4], p0, scale_h, ws);
-            add_pair_t<WEIGHTED>(acc[8 * i + 1], acc[8 * i + 5], p1, scale_h, ws);
-            add_pair_t<WEIGHTED>(acc[8 * i + 2], acc[8 * i + 6], p2, scale_h, ws);
-            add_pair_t<WEIGHTED>(acc[8 * i + 3], acc[8 * i + 7], p3, scale_h, ws);
+    for (int i = 0; i < NW; ++i) {
+        const uint32_t x = words[i];
+        if constexpr (TY == TBE_B200_INT8) {
+            fma2(acc[4 * i], acc[4 * i + 1], two(x & 0xFFu, x & 0xFF00u), s);
+            fma2(acc[4 * i + 2], acc[4 * i + 3], two(WEIGHTED ? (x >> 8) & 0xFF00u : x & 0xFF0000u, x >> 24), s);
+        } else {
+            const uint32_t y = x >> 24;
+            fma2(acc[8 * i], acc[8 * i + 1], two(x & 0xFu, x & 0xF0u), s);
+            fma2(acc[8 * i + 2], acc[8 * i + 3], two(x & 0xF00u, x & 0xF000u), s);
+            fma2(acc[8 * i + 4], acc[8 * i + 5], two(x & 0xF0000u, WEIGHTED ? (x >> 20) & 0xFu : x & 0xF00000u), s);
+            fma2(acc[8 * i + 6], acc[8 * i + 7], two(y & 0xFu, y & 0xF0u), s);
         }
     }
 }
@@ -437,7 +442,7 @@ __device__ __forceinline__ char* dest_segment(const LookupParams& p, int64_t b, 
 // (up to 32 floats per lane), the run's bag offsets, and the ring of rows in flight.
 constexpr int kPartBytes = kWarp * 128;
 constexpr int kMaxRunBags = 31;                        // bags of one run: their nb + 1 offsets are held one per lane
-constexpr int kRelBytes = 144;                         // (kMaxRunBags + 1) offsets, rounded to 16 bytes
+constexpr int kRelBytes = 160;                         // kMaxRunBags + 1 offsets and up to eight groups' bias sums
 #ifndef TBE_RING_BYTES
 #define TBE_RING_BYTES 4352                            // four stages of rows with up to 32 bytes per lane
 #endif
@@ -470,16 +475,10 @@ __host__ __device__ constexpr int min3(int a, int b, int c) { return a < b ? (a 
 // about to be consumed ended up waiting for loads that had just been issued.  A lane reads back only the bytes it
 // copied itself, so no barrier is involved.  A row that is not to be added (index -1, out of range, past the end
 // of the group's range) is zero-filled in the stage without being read.
-//
-// FOLD (INT8, unweighted, 16-bit output): the subtraction of the magic constant that turns a code into an fp16
-// value is skipped, (1024 + q) * scale is accumulated, and 1024 * sum(scale) is removed again at least every
-// 32 rows, which keeps the partial sums small enough for the extra term not to cost precision that a 16-bit
-// result could show.
-template <int TY, int LPR, int EPL, bool WEIGHTED, bool FOLD>
+template <int TY, int LPR, int EPL, bool WEIGHTED>
 __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
                                              uint32_t wsm)
 {
-    static_assert(!FOLD || (TY == TBE_B200_INT8 && !WEIGHTED), "the folded form is for unweighted INT8 pooling");
     static_assert(EPL == 16 || (EPL == 32 && (TY == TBE_B200_INT8 || TY == TBE_B200_INT4)), "32 elements per lane: INT8 / INT4 only");
     constexpr bool kHdr = (TY == TBE_B200_INT8 || TY == TBE_B200_INT4);
     constexpr bool k8 = (TY == TBE_B200_INT8);
@@ -561,37 +560,36 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
 #pragma unroll
     for (int s = 0; s < EPL; ++s) acc[s] = 0.0f;
     float bias_acc = 0.0f;
-    float scale_acc = 0.0f;   // sum of the row scales since the last fold (FOLD only)
-    int since_fold = 0;
-    (void)scale_acc;
-    (void)since_fold;
 
     char* const out0 = static_cast<char*>(p.output) + (b0 * p.out_stride + m.col) * ((p.out_ty == TBE_B200_FP32) ? 4 : 2);   // bag 0 of the run
     // Stores the finished bag `bag` of L rows (acc + bias_acc, times 1/L for MEAN).  Executed by whole groups.
     auto store_bag = [&](int bag, int L) {
         const float mm = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
         const float bm = bias_acc * mm;
+        auto pair = [&](int slot) {     // finished elements of slots `slot` (even) and slot + 1
+            return fma2_value(acc[slot], acc[slot + 1], mm * code_unit<TY, WEIGHTED>(slot), mm * code_unit<TY, WEIGHTED>(slot + 1), bm);
+        };
         // (computed here, once per bag, rather than kept in registers across the row loop)
         const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
         char* seg = p.dests ? dest_segment(p, b0 + bag, m.col, esz) : out0 + static_cast<int64_t>(bag) * (p.out_stride * esz);
         const bool vec = (reinterpret_cast<uintptr_t>(seg) & 15) == 0;
         bool stored = false;
-        if constexpr (FOLD) {
-            // Unweighted INT8 with a 16-bit output.  A unit's 16 elements start 4 elements before a 32-byte boundary.
+        if constexpr (k8) {
+            // INT8 with a 16-bit output.  A unit's 16 elements start 4 elements before a 32-byte boundary.
             // Its first 4 go to the unit before it (unit 0's, the row's tail, to the last unit), after which every
             // unit is 16 elements from a 32-byte boundary on: two aligned 16-byte stores, whole sectors.  The unit after
             // lane k's chunk c is lane k + 1's chunk c, or, for the last lane, lane 0's NEXT chunk.  `vec` is the same
             // for all lanes of the group, so the group takes the shuffles together.
-            if (vec) {
+            if (vec && esz == 2) {
                 uint32_t h[EPL / 2];
 #pragma unroll
                 for (int q = 0; q < EPL / 2; ++q) {
-                    const float lo16 = fmaf(acc[2 * q], mm, bm), hi16 = fmaf(acc[2 * q + 1], mm, bm);
+                    const float2 v = pair(2 * q);
                     if (p.out_ty == TBE_B200_FP16) {
-                        const __half2 hh = __floats2half2_rn(lo16, hi16);
+                        const __half2 hh = __floats2half2_rn(v.x, v.y);
                         h[q] = *reinterpret_cast<const uint32_t*>(&hh);
                     } else {
-                        const __nv_bfloat162 bb = __floats2bfloat162_rn(lo16, hi16);
+                        const __nv_bfloat162 bb = __floats2bfloat162_rn(v.x, v.y);
                         h[q] = *reinterpret_cast<const uint32_t*>(&bb);
                     }
                 }
@@ -615,9 +613,8 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
         if (!stored && act) {
 #pragma unroll
             for (int q = 0; q < EPL / 4; ++q) {
-                float v[4];
-#pragma unroll
-                for (int s = 0; s < 4; ++s) v[s] = fmaf(acc[4 * q + s], mm, bm);
+                const float2 a = pair(4 * q), b = pair(4 * q + 2);
+                const float v[4] = {a.x, a.y, b.x, b.y};
                 store_out<4>(seg, elem_of(4 * q), v, p.out_ty, vec);
             }
         }
@@ -626,16 +623,12 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     auto write_partial = [&]() {
 #pragma unroll
         for (int q = 0; q < EPL / 4; ++q)
-            sts16(wsm + static_cast<uint32_t>(q * kWarp + lane) * 16u, acc[4 * q + 0] + bias_acc, acc[4 * q + 1] + bias_acc,
-                  acc[4 * q + 2] + bias_acc, acc[4 * q + 3] + bias_acc);
+            sts16(wsm + static_cast<uint32_t>(q * kWarp + lane) * 16u, acc[4 * q + 0], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+        if (kHdr && k == 0) sts4(sm_rel + 4 * kWarp + 4 * g, __float_as_int(bias_acc));
     };
     // Finishes every bag that ends at the group's position (the one being summed, then the empty ones after it).
     auto drain = [&]() {
         while (pos == bag_end) {
-            if constexpr (FOLD) {
-                bias_acc = fmaf(-1024.0f, scale_acc, bias_acc);
-                scale_acc = 0.0f;
-            }
             if (bag_start < lo) write_partial();
             else store_bag(cur, bag_end - bag_start);
 #pragma unroll
@@ -729,9 +722,10 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
         if constexpr (kHdr) {
             const uint32_t hdr = __shfl_sync(kFull, r[0], 0, LPR);   // zero for a row that was not copied
             if (head_lane) r[0] = lds4(my_tail + st);                // the header lane's first HS slots: the row's tail
-            float ws;
-            const unsigned short scale_h = accum_header<WEIGHTED, FOLD>(hdr, w, ws, bias_acc, scale_acc);
-            accum_codes<TY, WEIGHTED, FOLD, NW>(r, scale_h, ws, acc);
+            // the header: fp16 scale, fp16 bias
+            const float sc = half_bits_to_float(hdr & 0xffffu), bi = half_bits_to_float(hdr >> 16);
+            bias_acc = WEIGHTED ? fmaf(bi, w, bias_acc) : bias_acc + bi;
+            accum_codes<TY, WEIGHTED, NW>(r, WEIGHTED ? sc * w : sc * kCodeScale, acc);
         } else if constexpr (TY == TBE_B200_FP8) {
             // byte -> fp32 by bit placement: ((b & 0x7f) << (16 + ebits)) as a float, times 2^(127 - bias),
             // sign bit or'ed in (reference: c310/op_kernel/common.h:120-167)
@@ -797,15 +791,6 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
             }
             request(st, __shfl_sync(kFull, idx_c, u, LPR));
         }
-        if constexpr (FOLD) {
-            since_fold += u_end;
-            if (since_fold + LPR > 32) {
-#pragma unroll
-                for (int s = 0; s < EPL; ++s) acc[s] = fmaf(-1024.0f, scale_acc, acc[s]);
-                scale_acc = 0.0f;
-                since_fold = 0;
-            }
-        }
     }
     cp_async_wait<0>();                    // nothing of this run is still on its way when the ring is handed on
 
@@ -813,15 +798,12 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     // owner's own piece, completed with the pieces of the groups after it.
     const bool open = active && bag_end >= 0 && bag_start < pos && pos < bag_end;
     if (open) {
-        if constexpr (FOLD) {
-            bias_acc = fmaf(-1024.0f, scale_acc, bias_acc);
-            scale_acc = 0.0f;
-        }
         if (bag_start < lo) write_partial();
     }
     __syncwarp();
     if (open && bag_start >= lo) {
         for (int gg = g + 1; gg < G && gg * per < bag_end; ++gg) {
+            if constexpr (kHdr) bias_acc += __int_as_float(lds4i(sm_rel + 4 * kWarp + 4 * gg));
 #pragma unroll
             for (int q = 0; q < EPL / 4; ++q) {
                 const float4 v = lds16f(wsm + static_cast<uint32_t>(q * kWarp + gg * LPR + k) * 16u);
@@ -835,7 +817,7 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     }
 }
 
-template <int TY, bool WEIGHTED, bool FOLD>
+template <int TY, bool WEIGHTED>
 __device__ __forceinline__ void pool_run_stream_by_width(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b,
                                                          int lane, uint32_t wsm)
 {
@@ -844,17 +826,17 @@ __device__ __forceinline__ void pool_run_stream_by_width(const LookupParams& p, 
     if constexpr (TY == TBE_B200_INT8 || TY == TBE_B200_INT4) {
         if (m.D >= 128 && (m.D & 31) == 0) {
             const int n32 = m.D / 32;
-            if (n32 <= 4) pool_run_stream<TY, 4, 32, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
-            else if (n32 <= 8) pool_run_stream<TY, 8, 32, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
-            else pool_run_stream<TY, 16, 32, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
+            if (n32 <= 4) pool_run_stream<TY, 4, 32, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+            else if (n32 <= 8) pool_run_stream<TY, 8, 32, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+            else pool_run_stream<TY, 16, 32, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
             return;
         }
     }
     const int nunits = m.D / 16;
-    if (nunits <= 4) pool_run_stream<TY, 4, 16, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
-    else if (nunits <= 8) pool_run_stream<TY, 8, 16, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
-    else if (nunits <= 16) pool_run_stream<TY, 16, 16, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
-    else pool_run_stream<TY, 32, 16, WEIGHTED, FOLD>(p, m, i0, nb, b, lane, wsm);
+    if (nunits <= 4) pool_run_stream<TY, 4, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+    else if (nunits <= 8) pool_run_stream<TY, 8, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+    else if (nunits <= 16) pool_run_stream<TY, 16, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+    else pool_run_stream<TY, 32, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
 }
 
 template <bool WEIGHTED>
@@ -863,18 +845,12 @@ __device__ __forceinline__ void pool_run_stream_by_type(const LookupParams& p, c
 {
     switch (m.ty) {
         case TBE_B200_INT8:
-            if constexpr (!WEIGHTED) {
-                if (p.out_ty != TBE_B200_FP32) {
-                    pool_run_stream_by_width<TBE_B200_INT8, false, true>(p, m, i0, nb, b, lane, wsm);
-                    return;
-                }
-            }
-            pool_run_stream_by_width<TBE_B200_INT8, WEIGHTED, false>(p, m, i0, nb, b, lane, wsm);
+            pool_run_stream_by_width<TBE_B200_INT8, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
             return;
-        case TBE_B200_INT4: pool_run_stream_by_width<TBE_B200_INT4, WEIGHTED, false>(p, m, i0, nb, b, lane, wsm); return;
-        case TBE_B200_FP8: pool_run_stream_by_width<TBE_B200_FP8, WEIGHTED, false>(p, m, i0, nb, b, lane, wsm); return;
-        case TBE_B200_FP16: pool_run_stream_by_width<TBE_B200_FP16, WEIGHTED, false>(p, m, i0, nb, b, lane, wsm); return;
-        default: pool_run_stream_by_width<TBE_B200_FP32, WEIGHTED, false>(p, m, i0, nb, b, lane, wsm); return;
+        case TBE_B200_INT4: pool_run_stream_by_width<TBE_B200_INT4, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
+        case TBE_B200_FP8: pool_run_stream_by_width<TBE_B200_FP8, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
+        case TBE_B200_FP16: pool_run_stream_by_width<TBE_B200_FP16, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
+        default: pool_run_stream_by_width<TBE_B200_FP32, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
     }
 }
 
@@ -888,41 +864,11 @@ __device__ __forceinline__ void pool_run_stream_by_type(const LookupParams& p, c
 // pool_run_stream runs its end of a bag once per bag AND lane group.  No row of another bag shares a step, so
 // nothing is masked: a step's missing rows are zero-filled.
 //
-// What bounds the pooled lookup is the instructions issued per row, so the arithmetic is cut as well.  A code is used where
-// it lies: masked out of its word and read as fp32 it is a subnormal (q * 2^8 * 2^-149 for the second byte), which is
-// exact, and so is its product with the row's scale times 2^111; packed fp32 FMAs (two elements each) add the
-// products with one rounding, as before.  What the place of a code multiplies is undone when the bag is stored.  One mask
-// and half an FMA per code instead of a permute and an FMA, one mask instead of three instructions for an INT4 code.
-// With per-sample weights scale * weight may have any magnitude, so the codes are made ordinary numbers first (2^23 + q in
-// one masking instruction, less 2^23 in half a packed addition).
-//
 // Row fetch.  Rows travel through a ring of NS stages in the warp's shared memory with asynchronous copies through L1, each
 // lane copying and reading back only its own bytes.  CB bytes per lane and row: 4, 8, 16 or 32, so that narrow rows keep
 // all lanes busy and one pass covers up to 256 bytes (INT4: 128); wider rows take several passes over the run, each
 // over its own columns.  Any D that is a multiple of 4 will do: a row's last unit may reach into the row's padding,
 // whose sums are not stored.
-
-// Two packed fp32 numbers, and c += a * b and a + b on them.
-__device__ __forceinline__ unsigned long long pack2(uint32_t lo, uint32_t hi)
-{
-    unsigned long long v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
-    return v;
-}
-__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long v;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
-}
-__device__ __forceinline__ void sts16u(uint32_t a, unsigned long long x, unsigned long long y)
-{
-    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
-}
 
 // Asynchronous 4-byte copy by the lanes that `on` selects, predicated instead of branched around.
 __device__ __forceinline__ void cp_async4_if(bool on, uint32_t dst, const void* src, int bytes)
@@ -1003,9 +949,8 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
     const uint64_t rows_avail = static_cast<uint64_t>(m.avail) / stride;
     const uint64_t max_rows = rows_avail < 0x80000000ull ? rows_avail : 0x80000000ull;
     const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
-    constexpr float kScaleUp = 0x1p111f, kUnit = 0x1p-38f;              // unweighted codes: 2^-149 * 2^111
     constexpr float kFp8W = 0x1p60f;                                    // weighted FP8: so much of fp8_mult is in the weights
-    const float mul_base = kHdr ? (WEIGHTED ? 1.0f : 1.0f / kUnit) : kF8 ? (WEIGHTED ? p.fp8_mult / kFp8W : p.fp8_mult) : 1.0f;
+    const float mul_base = kF8 ? (WEIGHTED ? p.fp8_mult / kFp8W : p.fp8_mult) : 1.0f;
 
     for (int u0 = 0; u0 < units; u0 += 8 * NCH) {
         const bool first_pass = (u0 == 0);
@@ -1015,9 +960,9 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
         const uint8_t* side_base = m.table + (first_pass ? payload : 0);
         const int size0 = u0 + g < units ? CHB : 0, size1 = u0 + g + 8 < units ? CHB : 0;
 
-        unsigned long long acc[2 * NQ];                // pairs of elements; 0 is (0.0f, 0.0f)
+        float acc[4 * NQ];
 #pragma unroll
-        for (int i = 0; i < 2 * NQ; ++i) acc[i] = 0ull;
+        for (int i = 0; i < 4 * NQ; ++i) acc[i] = 0.0f;
         float bias_acc = 0.0f;
 
         // Indices are loaded 32 at a time, two chunks ahead, kept as loaded until their chunk's turn (anything computed from
@@ -1067,55 +1012,26 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
             if constexpr (kHdr) {
                 const float sc = half_bits_to_float(hdr & 0xffffu), bi = half_bits_to_float(hdr >> 16);
                 bias_acc = WEIGHTED ? fmaf(bi, w, bias_acc) : bias_acc + bi;
-                const uint32_t s = __float_as_uint(WEIGHTED ? sc * w : sc * kScaleUp);
-                const unsigned long long ss = pack2(s, s);
-                // 2^23 + q when the codes are to be ordinary numbers
-                constexpr uint32_t kM = WEIGHTED ? 0x4B000000u : 0u;
-                const unsigned long long minus = pack2(0xCB000000u, 0xCB000000u);
-                auto two = [&](uint32_t a, uint32_t b) { return WEIGHTED ? add2(pack2(a, b), minus) : pack2(a, b); };
-#pragma unroll
-                for (int i = 0; i < NW; ++i) {
-                    const uint32_t x = r[i];
-                    if constexpr (k8) {
-                        fma2(acc[2 * i], two((x & 0xFFu) | kM, (x & 0xFF00u) | kM), ss);
-                        fma2(acc[2 * i + 1], two((x & 0xFF0000u) >> (WEIGHTED ? 8 : 0) | kM, (x >> 24) | kM), ss);
-                    } else {
-                        const uint32_t y = x >> 24;
-                        fma2(acc[4 * i], two((x & 0xFu) | kM, (x & 0xF0u) | kM), ss);
-                        fma2(acc[4 * i + 1], two((x & 0xF00u) | kM, (x & 0xF000u) | kM), ss);
-                        fma2(acc[4 * i + 2], two((x & 0xF0000u) | kM, (WEIGHTED ? (x >> 20) & 0xFu : x & 0xF00000u) | kM), ss);
-                        fma2(acc[4 * i + 3], two((y & 0xFu) | kM, (y & 0xF0u) | kM), ss);
-                    }
-                }
+                accum_codes<TY, WEIGHTED, NW>(r, WEIGHTED ? sc * w : sc * kCodeScale, acc);
             } else if constexpr (kF8) {
                 // byte -> bf16, two at a time: sign to the top, the rest to exponent and mantissa; a bf16 is the upper half of an fp32
                 const uint32_t sh = p.fp8_shift - 16;
-                const uint32_t s = __float_as_uint(WEIGHTED ? w * kFp8W : 1.0f);
-                const unsigned long long ss = pack2(s, s);
+                const float s = WEIGHTED ? w * kFp8W : 1.0f;
 #pragma unroll
                 for (int i = 0; i < NW; ++i) {
                     const uint32_t x = r[i], y = x >> 8;
                     const uint32_t even = ((x & 0x007F007Fu) << sh) | ((x & 0x00800080u) << 8), odd = ((y & 0x007F007Fu) << sh) | ((y & 0x00800080u) << 8);
-                    fma2(acc[2 * i], pack2(even << 16, odd << 16), ss);
-                    fma2(acc[2 * i + 1], pack2(even & 0xffff0000u, odd & 0xffff0000u), ss);
+                    fma2(acc[4 * i], acc[4 * i + 1], pack2(even << 16, odd << 16), s);
+                    fma2(acc[4 * i + 2], acc[4 * i + 3], pack2(even & 0xffff0000u, odd & 0xffff0000u), s);
                 }
             } else if constexpr (k32) {
-                const uint32_t s = __float_as_uint(w);
-                const unsigned long long ss = pack2(s, s);
 #pragma unroll
-                for (int i = 0; i < NW / 2; ++i) {
-                    if constexpr (WEIGHTED) fma2(acc[i], pack2(r[2 * i], r[2 * i + 1]), ss);
-                    else acc[i] = add2(acc[i], pack2(r[2 * i], r[2 * i + 1]));
-                }
+                for (int i = 0; i < NW / 2; ++i) fma2(acc[2 * i], acc[2 * i + 1], pack2(r[2 * i], r[2 * i + 1]), w);
             } else {
-                const uint32_t s = __float_as_uint(w);
-                const unsigned long long ss = pack2(s, s);
 #pragma unroll
                 for (int i = 0; i < NW; ++i) {
                     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[i]));
-                    const unsigned long long v = pack2(__float_as_uint(f.x), __float_as_uint(f.y));
-                    if constexpr (WEIGHTED) fma2(acc[i], v, ss);
-                    else acc[i] = add2(acc[i], v);
+                    fma2(acc[2 * i], acc[2 * i + 1], pack2(__float_as_uint(f.x), __float_as_uint(f.y)), w);
                 }
             }
         };
@@ -1181,24 +1097,19 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
             for (int x0 = 0; x0 < NQ; x0 += XQ) {
                 __syncwarp();                          // the previous exchange has been read
 #pragma unroll
-                for (int i = 0; i < XQ; ++i) sts16u(sm_x + static_cast<uint32_t>(i * XROW + lane) * 16u, acc[2 * (x0 + i)], acc[2 * (x0 + i) + 1]);
+                for (int i = 0; i < XQ; ++i)
+                    sts16(sm_x + static_cast<uint32_t>(i * XROW + lane) * 16u, acc[4 * (x0 + i)], acc[4 * (x0 + i) + 1], acc[4 * (x0 + i) + 2], acc[4 * (x0 + i) + 3]);
                 __syncwarp();
                 const int xu = lane / XQ, q = x0 + lane % XQ;     // the unit (of eight) and the quad this lane finishes
                 if (xu < 8) {
                     const uint32_t from = sm_x + static_cast<uint32_t>((lane % XQ) * XROW + xu) * 16u;
                     const float4 a = lds16f(from), b = lds16f(from + 128), c = lds16f(from + 256), d = lds16f(from + 384);
                     // what a code's place in its word multiplied
-                    float m0 = mul, m1 = mul, m2 = mul, m3 = mul;
-                    if constexpr (k8) {
-                        m1 = mul * 0x1p-8f;
-                        m2 = WEIGHTED ? m1 : mul * 0x1p-16f;
-                    } else if constexpr (k4) {
-                        const bool upper = q & 1;      // nibbles 4 .. 7 of the word
-                        m0 = upper ? mul * 0x1p-16f : mul;
-                        m1 = upper ? (WEIGHTED ? mul : mul * 0x1p-20f) : mul * 0x1p-4f;
-                        m2 = upper ? mul : mul * 0x1p-8f;
-                        m3 = upper ? mul * 0x1p-4f : mul * 0x1p-12f;
-                    }
+                    const bool upper = k4 && (q & 1);  // nibbles 4 .. 7 of the word
+                    const float m0 = mul * (upper ? code_unit<TY, WEIGHTED>(4) : code_unit<TY, WEIGHTED>(0));
+                    const float m1 = mul * (upper ? code_unit<TY, WEIGHTED>(5) : code_unit<TY, WEIGHTED>(1));
+                    const float m2 = mul * (upper ? code_unit<TY, WEIGHTED>(6) : code_unit<TY, WEIGHTED>(2));
+                    const float m3 = mul * (upper ? code_unit<TY, WEIGHTED>(7) : code_unit<TY, WEIGHTED>(3));
                     const float v[4] = {fmaf((a.x + b.x) + (c.x + d.x), m0, bm), fmaf((a.y + b.y) + (c.y + d.y), m1, bm),
                                         fmaf((a.z + b.z) + (c.z + d.z), m2, bm), fmaf((a.w + b.w) + (c.w + d.w), m3, bm)};
                     constexpr int QPU = EPU / 4;       // quads of a unit
@@ -1209,7 +1120,7 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 2 * NQ; ++i) acc[i] = 0ull;
+            for (int i = 0; i < 4 * NQ; ++i) acc[i] = 0.0f;
             bias_acc = 0.0f;
         };
 
@@ -1393,7 +1304,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe
                              (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32 ||
                               (m.ty == TBE_B200_FP8 && p.fp8_shift <= 23));
         // Widths that give every lane of a row the same 16 elements go through the streams, which issue a third fewer instructions
-        // there (64 INT8 tables of 128: 3.83 ms against 6.0 in steps; INT4 of 64/128/256: 1.52 against 1.91 ms); all others in
+        // there (64 INT8 tables of 128: 3.74 ms against 6.0 in steps; INT4 of 64/128/256: 1.30 against 1.91 ms); all others in
         // steps (16 tables of 20 to 1024 elements of four types: 194 us; 342 us one bag at a time or byte by byte).
         if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
         else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
