@@ -422,6 +422,25 @@ __device__ __forceinline__ void accum_codes(const uint32_t (&words)[NW], float s
     }
 }
 
+// Adds NW 32-bit words of FP8 bytes times `s`, two bytes at a time as bf16: sign to the top, the rest to exponent and
+// mantissa (reference: c310/op_kernel/common.h:120-167); a bf16 is the upper half of an fp32.  The sums lack a factor of
+// fp8_mult; with per-sample weights kFp8Weight of it is in `s`, so that neither the products nor the weights leave fp32's range.
+// 16 tables of 128 FP8, batch 8192: 212 -> 165 us against placing, scaling and signing every byte by itself (D = 256 with
+// weights: 426 -> 316).
+constexpr float kFp8Weight = 0x1p60f;
+template <int NW>
+__device__ __forceinline__ void accum_fp8(const uint32_t (&words)[NW], uint32_t fp8_shift, float s, float* acc)
+{
+    const uint32_t sh = fp8_shift - 16;                // exponent bits
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        const uint32_t x = words[i], y = x >> 8;
+        const uint32_t even = ((x & 0x007F007Fu) << sh) | ((x & 0x00800080u) << 8), odd = ((y & 0x007F007Fu) << sh) | ((y & 0x00800080u) << 8);
+        fma2(acc[4 * i], acc[4 * i + 1], pack2(even << 16, odd << 16), s);
+        fma2(acc[4 * i + 2], acc[4 * i + 3], pack2(even & 0xffff0000u, odd & 0xffff0000u), s);
+    }
+}
+
 // Output address of element 0 of bag `b` of the table at column `col`, when the result is scattered
 // over per-destination buffers (bag b belongs to destination b / rows_per_dest).
 __device__ __forceinline__ char* dest_segment(const LookupParams& p, int64_t b, int64_t col, int esz)
@@ -566,8 +585,9 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     auto store_bag = [&](int bag, int L) {
         const float mm = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
         const float bm = bias_acc * mm;
+        const float mul = TY == TBE_B200_FP8 ? mm * (WEIGHTED ? p.fp8_mult / kFp8Weight : p.fp8_mult) : mm;
         auto pair = [&](int slot) {     // finished elements of slots `slot` (even) and slot + 1
-            return fma2_value(acc[slot], acc[slot + 1], mm * code_unit<TY, WEIGHTED>(slot), mm * code_unit<TY, WEIGHTED>(slot + 1), bm);
+            return fma2_value(acc[slot], acc[slot + 1], mul * code_unit<TY, WEIGHTED>(slot), mul * code_unit<TY, WEIGHTED>(slot + 1), bm);
         };
         // (computed here, once per bag, rather than kept in registers across the row loop)
         const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
@@ -727,25 +747,20 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
             bias_acc = WEIGHTED ? fmaf(bi, w, bias_acc) : bias_acc + bi;
             accum_codes<TY, WEIGHTED, NW>(r, WEIGHTED ? sc * w : sc * kCodeScale, acc);
         } else if constexpr (TY == TBE_B200_FP8) {
-            // byte -> fp32 by bit placement: ((b & 0x7f) << (16 + ebits)) as a float, times 2^(127 - bias),
-            // sign bit or'ed in (reference: c310/op_kernel/common.h:120-167)
+            accum_fp8<NW>(r, p.fp8_shift, WEIGHTED ? w * kFp8Weight : 1.0f, acc);
+        } else if constexpr (TY == TBE_B200_FP16 && !WEIGHTED) {
+            // value * 1.0 + acc in one mixed FMA
 #pragma unroll
-            for (int i4 = 0; i4 < 4; ++i4) {
-#pragma unroll
-                for (int b4 = 0; b4 < 4; ++b4) {
-                    const uint32_t by = (r[i4] >> (8 * b4)) & 0xffu;
-                    const float mag = __uint_as_float((by & 0x7fu) << p.fp8_shift) * p.fp8_mult;
-                    const float val = __uint_as_float(__float_as_uint(mag) | ((by & 0x80u) << 24));
-                    acc[4 * i4 + b4] = fmaf(w, val, acc[4 * i4 + b4]);
-                }
-            }
+            for (int i8 = 0; i8 < 8; ++i8) add_pair_t<false>(acc[2 * i8], acc[2 * i8 + 1], r[i8], 0x3c00u, w);
         } else if constexpr (TY == TBE_B200_FP16) {
-            // unweighted: value * 1.0 + acc in one mixed FMA
 #pragma unroll
-            for (int i8 = 0; i8 < 8; ++i8) add_pair_t<WEIGHTED>(acc[2 * i8], acc[2 * i8 + 1], r[i8], 0x3c00u, w);
+            for (int i8 = 0; i8 < 8; ++i8) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[i8]));
+                fma2(acc[2 * i8], acc[2 * i8 + 1], pack2(__float_as_uint(f.x), __float_as_uint(f.y)), w);
+            }
         } else {
 #pragma unroll
-            for (int s = 0; s < 16; ++s) acc[s] = fmaf(w, __uint_as_float(r[s]), acc[s]);
+            for (int s = 0; s < 8; ++s) fma2(acc[2 * s], acc[2 * s + 1], pack2(r[2 * s], r[2 * s + 1]), w);
         }
     };
 
@@ -949,8 +964,7 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
     const uint64_t rows_avail = static_cast<uint64_t>(m.avail) / stride;
     const uint64_t max_rows = rows_avail < 0x80000000ull ? rows_avail : 0x80000000ull;
     const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
-    constexpr float kFp8W = 0x1p60f;                                    // weighted FP8: so much of fp8_mult is in the weights
-    const float mul_base = kF8 ? (WEIGHTED ? p.fp8_mult / kFp8W : p.fp8_mult) : 1.0f;
+    const float mul_base = kF8 ? (WEIGHTED ? p.fp8_mult / kFp8Weight : p.fp8_mult) : 1.0f;
 
     for (int u0 = 0; u0 < units; u0 += 8 * NCH) {
         const bool first_pass = (u0 == 0);
@@ -1014,16 +1028,7 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
                 bias_acc = WEIGHTED ? fmaf(bi, w, bias_acc) : bias_acc + bi;
                 accum_codes<TY, WEIGHTED, NW>(r, WEIGHTED ? sc * w : sc * kCodeScale, acc);
             } else if constexpr (kF8) {
-                // byte -> bf16, two at a time: sign to the top, the rest to exponent and mantissa; a bf16 is the upper half of an fp32
-                const uint32_t sh = p.fp8_shift - 16;
-                const float s = WEIGHTED ? w * kFp8W : 1.0f;
-#pragma unroll
-                for (int i = 0; i < NW; ++i) {
-                    const uint32_t x = r[i], y = x >> 8;
-                    const uint32_t even = ((x & 0x007F007Fu) << sh) | ((x & 0x00800080u) << 8), odd = ((y & 0x007F007Fu) << sh) | ((y & 0x00800080u) << 8);
-                    fma2(acc[4 * i], acc[4 * i + 1], pack2(even << 16, odd << 16), s);
-                    fma2(acc[4 * i + 2], acc[4 * i + 3], pack2(even & 0xffff0000u, odd & 0xffff0000u), s);
-                }
+                accum_fp8<NW>(r, p.fp8_shift, WEIGHTED ? w * kFp8Weight : 1.0f, acc);
             } else if constexpr (k32) {
 #pragma unroll
                 for (int i = 0; i < NW / 2; ++i) fma2(acc[2 * i], acc[2 * i + 1], pack2(r[2 * i], r[2 * i + 1]), w);
