@@ -29,7 +29,7 @@ CABI_LIB = os.path.join(LIB_DIR, "libtbe_b200.so")
 TORCH_LIB = os.path.join(LIB_DIR, "libtbe_b200_torch.so")
 
 CUDA_SOURCES = ["tbe_common.cu", "tbe_lookup.cu", "tbe_quant.cu", "tbe_permute.cu", "tbe_sparse.cu", "tbe_exchange.cu"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "--split-compile=0", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
+NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "-I" + INCLUDE]
 
 
