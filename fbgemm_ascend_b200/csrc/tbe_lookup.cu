@@ -386,7 +386,7 @@ __device__ __forceinline__ float2 fma2_value(float a0, float a1, float b0, float
 // multiplied is undone when the bag is stored (code_unit).  With per-sample weights scale * weight may have any magnitude, so
 // the codes are made ordinary numbers first: 2^23 + q in the masking instruction, less 2^23 in half a packed addition.
 // A step of eight 128-byte rows takes 162 instructions instead of 177 with a byte permute and a mixed FMA per code: 64 INT8
-// tables of 128, batch 65536: 3.83 -> 3.74 ms; INT4 of 64/128/256: 1.52 -> 1.30 ms.
+// tables of 128, batch 65536: 3.83 -> 3.78 ms; INT4 of 64/128/256: 1.52 -> 1.41 ms.
 constexpr float kCodeScale = 0x1p111f;
 template <int TY, bool WEIGHTED>
 __device__ constexpr float code_unit(int slot)
@@ -1309,8 +1309,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe
                              (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32 ||
                               (m.ty == TBE_B200_FP8 && p.fp8_shift <= 23));
         // Widths that give every lane of a row the same 16 elements go through the streams, which issue a third fewer instructions
-        // there (64 INT8 tables of 128: 3.74 ms against 6.0 in steps; INT4 of 64/128/256: 1.30 against 1.91 ms); all others in
-        // steps (16 tables of 20 to 1024 elements of four types: 194 us; 342 us one bag at a time or byte by byte).
+        // there (64 INT8 tables of 128: 3.78 ms against 6.0 in steps; INT4 of 64/128/256: 1.41 against 1.91 ms); all others in
+        // steps (16 tables of 20 to 1024 elements of four types: 174 us; 338 us one bag at a time or byte by byte).
         if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
         else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
         else if (m.D > 0 && p.idx64) pool_run_bytewise<int64_t>(p, m, i, nb, b, lane);
