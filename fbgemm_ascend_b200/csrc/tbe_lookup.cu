@@ -1312,7 +1312,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe
                              (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32 ||
                               (m.ty == TBE_B200_FP8 && p.fp8_shift <= 23));
         // Widths that give every lane of a row the same 16 elements go through the streams, which issue a third fewer instructions
-        // there (64 INT8 tables of 128: 3.78 ms against 6.0 in steps; INT4 of 64/128/256: 1.41 against 1.91 ms); all others in
+        // there (64 INT8 tables of 128: 3.63 ms against 6.0 in steps; INT4 of 64/128/256: 1.23 against 1.91 ms); all others in
         // steps (16 tables of 20 to 1024 elements of four types: 174 us; 338 us one bag at a time or byte by byte).
         if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
         else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
