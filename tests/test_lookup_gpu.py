@@ -395,8 +395,8 @@ def test_row_widths_at_the_edges_of_the_units(weights_ty, dims, weighted, out_ty
         assert np.all(np.abs(got - want) <= bound), f"max excess {(np.abs(got - want) - bound).max()}"
 
 
-@pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4])
-@pytest.mark.parametrize("magnitude", [1e-30, 1e-12, 1.0, 1e12])
+@pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4, O.FP8])
+@pytest.mark.parametrize("magnitude", [1e-30, 1e-12, 1.0, 1e12, 1e25])
 def test_weights_of_any_magnitude(weights_ty, magnitude):
     """Per-sample weights far from one, next to bags of ordinary ones: relative to the magnitudes that go in, the result
     is as good as with weights around one."""
@@ -444,3 +444,13 @@ def test_sequence_rows_of_any_width(weights_ty, dims, out_ty):
     for ds in (dims, dims[:2]):
         c = make_case(rng, [weights_ty] * len(ds), ds, [70] * len(ds), 2, lens[:2 * len(ds)], np.int64, False, prune_frac=0.05)
         run(c, O.NONE, out_ty, f"sequence dims={ds}")
+
+
+@pytest.mark.parametrize("fp8", [(5, 15), (3, 3), (2, 1), (7, 63)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_fp8_formats(fp8, weighted):
+    """FP8 rows of other exponent widths and biases, in streams (64, 128, 256) and in steps of eight rows (36, 260)."""
+    rng = np.random.default_rng(seed_of("fp8", fp8, weighted))
+    c = make_case(rng, [O.FP8] * 5, [64, 36, 128, 260, 256], [60] * 5, 7, rng.integers(0, 30, 35), np.int32, weighted, prune_frac=0.03)
+    run(c, O.SUM, O.FP32, f"fp8={fp8}", fp8=fp8)
+    run(c, O.MEAN, O.FP16, f"fp8={fp8}", fp8=fp8)
