@@ -396,10 +396,10 @@ def test_row_widths_at_the_edges_of_the_units(weights_ty, dims, weighted, out_ty
 
 
 @pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4, O.FP8])
-@pytest.mark.parametrize("magnitude", [1e-30, 1e-12, 1.0, 1e12, 1e25])
+@pytest.mark.parametrize("magnitude", [1e-30, 1e-12, 1.0, 1e12, 1e25, 1e37])
 def test_weights_of_any_magnitude(weights_ty, magnitude):
     """Per-sample weights far from one, next to bags of ordinary ones: relative to the magnitudes that go in, the result
-    is as good as with weights around one."""
+    is as good as with weights around one.  (The largest sums of magnitudes here are about 1e38.)"""
     rng = np.random.default_rng(17)
     c = make_case(rng, [weights_ty] * 2, [64, 264], [80, 90], 9, rng.integers(0, 40, 18), np.int64, True)
     c.weights[: int(c.offsets[7])] *= np.float32(magnitude)
