@@ -479,7 +479,7 @@ __device__ __forceinline__ char* dest_segment(const LookupParams& p, int64_t b, 
 // (up to 32 floats per lane), the run's bag offsets, and the ring of rows in flight.
 constexpr int kPartBytes = kWarp * 128;
 constexpr int kMaxRunBags = 31;                        // bags of one run: their nb + 1 offsets are held one per lane
-constexpr int kRelBytes = 160;                         // kMaxRunBags + 1 offsets and up to eight groups' bias sums
+constexpr int kRelBytes = 128;                         // kMaxRunBags + 1 offsets
 #ifndef TBE_RING_BYTES
 #define TBE_RING_BYTES 4352                            // four stages of rows with up to 32 bytes per lane
 #endif
@@ -599,14 +599,32 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     float bias_acc = 0.0f;
 
     char* const out0 = static_cast<char*>(p.output) + (b0 * p.out_stride + m.col) * ((p.out_ty == TBE_B200_FP32) ? 4 : 2);   // bag 0 of the run
-    // Stores the finished bag `bag` of L rows (acc + bias_acc, times 1/L for MEAN).  Executed by whole groups.
+    // Makes sums of elements of the sums of codes (or of placed FP8 bytes): what their place multiplied is undone and the
+    // biases are added.  Done before a bag is stored and before a piece of one is handed over: the codes of a piece are
+    // many times what is left of them beside their biases, and would round the other pieces' sums away.
+    auto settle = [&]() {
+        if constexpr (kHdr || (TY == TBE_B200_FP8 && !WEIGHTED)) {
+#pragma unroll
+            for (int s = 0; s < EPL; s += 2) {
+                const float u0 = TY == TBE_B200_FP8 ? p.fp8_mult : code_unit<TY, WEIGHTED>(s);
+                const float u1 = TY == TBE_B200_FP8 ? p.fp8_mult : code_unit<TY, WEIGHTED>(s + 1);
+                const float2 v = fma2_value(acc[s], acc[s + 1], u0, u1, bias_acc);
+                acc[s] = v.x;
+                acc[s + 1] = v.y;
+            }
+        }
+    };
+    // Stores the settled bag `bag` of L rows (times 1/L for MEAN).  Executed by whole groups.
     auto store_bag = [&](int bag, int L) {
-        const float mm = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
-        const float bm = bias_acc * mm;
-        const float mul = TY == TBE_B200_FP8 && !WEIGHTED ? mm * p.fp8_mult : mm;
-        auto pair = [&](int slot) {     // finished elements of slots `slot` (even) and slot + 1
-            return fma2_value(acc[slot], acc[slot + 1], mul * code_unit<TY, WEIGHTED>(slot), mul * code_unit<TY, WEIGHTED>(slot + 1), bm);
-        };
+        if (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) {
+            const float mm = 1.0f / static_cast<float>(L);
+#pragma unroll
+            for (int s = 0; s < EPL; s += 2) {
+                const float2 v = fma2_value(acc[s], acc[s + 1], mm, mm, 0.0f);
+                acc[s] = v.x;
+                acc[s + 1] = v.y;
+            }
+        }
         // (computed here, once per bag, rather than kept in registers across the row loop)
         const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
         char* seg = p.dests ? dest_segment(p, b0 + bag, m.col, esz) : out0 + static_cast<int64_t>(bag) * (p.out_stride * esz);
@@ -622,12 +640,11 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
                 uint32_t h[EPL / 2];
 #pragma unroll
                 for (int q = 0; q < EPL / 2; ++q) {
-                    const float2 v = pair(2 * q);
                     if (p.out_ty == TBE_B200_FP16) {
-                        const __half2 hh = __floats2half2_rn(v.x, v.y);
+                        const __half2 hh = __floats2half2_rn(acc[2 * q], acc[2 * q + 1]);
                         h[q] = *reinterpret_cast<const uint32_t*>(&hh);
                     } else {
-                        const __nv_bfloat162 bb = __floats2bfloat162_rn(v.x, v.y);
+                        const __nv_bfloat162 bb = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
                         h[q] = *reinterpret_cast<const uint32_t*>(&bb);
                     }
                 }
@@ -650,23 +667,19 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
         }
         if (!stored && act) {
 #pragma unroll
-            for (int q = 0; q < EPL / 4; ++q) {
-                const float2 a = pair(4 * q), b = pair(4 * q + 2);
-                const float v[4] = {a.x, a.y, b.x, b.y};
-                store_out<4>(seg, elem_of(4 * q), v, p.out_ty, vec);
-            }
+            for (int q = 0; q < EPL / 4; ++q) store_out<4>(seg, elem_of(4 * q), &acc[4 * q], p.out_ty, vec);
         }
     };
-    // Hands this group's piece of a bag that started in an earlier group's range to that bag's owner.
+    // Hands this group's settled piece of a bag that started in an earlier group's range to that bag's owner.
     auto write_partial = [&]() {
 #pragma unroll
         for (int q = 0; q < EPL / 4; ++q)
             sts16(wsm + static_cast<uint32_t>(q * kWarp + lane) * 16u, acc[4 * q + 0], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-        if (kHdr && k == 0) sts4(sm_rel + 4 * kWarp + 4 * g, __float_as_int(bias_acc));
     };
     // Finishes every bag that ends at the group's position (the one being summed, then the empty ones after it).
     auto drain = [&]() {
         while (pos == bag_end) {
+            settle();
             if (bag_start < lo) write_partial();
             else store_bag(cur, bag_end - bag_start);
 #pragma unroll
@@ -831,12 +844,12 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     // owner's own piece, completed with the pieces of the groups after it.
     const bool open = active && bag_end >= 0 && bag_start < pos && pos < bag_end;
     if (open) {
+        settle();
         if (bag_start < lo) write_partial();
     }
     __syncwarp();
     if (open && bag_start >= lo) {
         for (int gg = g + 1; gg < G && gg * per < bag_end; ++gg) {
-            if constexpr (kHdr) bias_acc += __int_as_float(lds4i(sm_rel + 4 * kWarp + 4 * gg));
 #pragma unroll
             for (int q = 0; q < EPL / 4; ++q) {
                 const float4 v = lds16f(wsm + static_cast<uint32_t>(q * kWarp + gg * LPR + k) * 16u);

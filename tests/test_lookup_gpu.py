@@ -454,3 +454,30 @@ def test_fp8_formats(fp8, weighted):
     c = make_case(rng, [O.FP8] * 5, [64, 36, 128, 260, 256], [60] * 5, 7, rng.integers(0, 30, 35), np.int32, weighted, prune_frac=0.03)
     run(c, O.SUM, O.FP32, f"fp8={fp8}", fp8=fp8)
     run(c, O.MEAN, O.FP16, f"fp8={fp8}", fp8=fp8)
+
+
+def _one_table_of_rows(ty, D, headers, codes, idx, offsets, B, weights=None):
+    """A table whose row r has the fp16 pair headers[r] and the codes codes[r]."""
+    rb = O.row_bytes(ty, D, 16)
+    rows = np.zeros((len(headers), rb), np.uint8)
+    for r, (scale, bias) in enumerate(headers):
+        rows[r, :4] = np.frombuffer(np.array([scale, bias], np.float16).tobytes(), np.uint8)
+        q = np.asarray(codes[r], np.uint8)
+        rows[r, 4:4 + (D if ty == O.INT8 else D // 2)] = q if ty == O.INT8 else q[0::2] | (q[1::2] << 4)
+    dev, wo, wt, do = O.concat_tables([rows], [ty], [D])
+    return Case(dev, wo, wt, do, np.asarray(idx, np.int32), np.asarray(offsets, np.int32), weights, [ty], [D], [len(headers)], B)
+
+
+@pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4])
+@pytest.mark.parametrize("D", [64, 128, 256, 512])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_pieces_of_a_bag_are_added_without_their_cancelled_parts(weights_ty, D, weighted):
+    """A bag of 64 rows that several lane groups sum: 32 rows of code * 2^-10, then 32 rows of code * scale - 32768 = 0 with
+    code * scale = 32768.  Every lane group has rows of one kind only (2, 4 or 8 equal ranges), every sum is a multiple of
+    2^-10 below 2^13 or of 2^15 below 2^21, so nothing rounds as long as the pieces are handed over with their
+    biases: the result is exact.  With the codes' sums added first, 2^20 would take the bits below 2^-3 away."""
+    small = np.arange(D) % (255 if weights_ty == O.INT8 else 15) + 1
+    big = 64 if weights_ty == O.INT8 else 8
+    c = _one_table_of_rows(weights_ty, D, [(2.0 ** -10, 0.0), (32768.0 / big, -32768.0)], [small, np.full(D, big)],
+                           [0] * 32 + [1] * 32, [0, 64], 1, np.ones(64, np.float32) if weighted else None)
+    assert np.array_equal(gpu_lookup(c, O.SUM, O.FP32)[0], (small * 2.0 ** -5).astype(np.float32))
