@@ -995,7 +995,7 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
     const uint64_t rows_avail = static_cast<uint64_t>(m.avail) / stride;
     const uint64_t max_rows = rows_avail < 0x80000000ull ? rows_avail : 0x80000000ull;
     const int esz = (p.out_ty == TBE_B200_FP32) ? 4 : 2;
-    const float mul_base = kF8 && !WEIGHTED ? p.fp8_mult : 1.0f;
+    const float unit_base = kF8 && !WEIGHTED ? p.fp8_mult : 1.0f;
 
     for (int u0 = 0; u0 < units; u0 += 8 * NCH) {
         const bool first_pass = (u0 == 0);
@@ -1126,7 +1126,6 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
             bias_acc += __shfl_xor_sync(kFull, bias_acc, 8);
             bias_acc += __shfl_xor_sync(kFull, bias_acc, 16);
             const float mm = (p.pooling_mode == TBE_B200_POOL_MEAN && L > 0) ? 1.0f / static_cast<float>(L) : 1.0f;
-            const float mul = mul_base * mm, bm = bias_acc * mm;
             char* seg = p.dests ? dest_segment(p, b0 + bag, m.col, esz) : static_cast<char*>(p.output) + ((b0 + bag) * p.out_stride + m.col) * esz;
             const bool vec = (reinterpret_cast<uintptr_t>(seg) & (4 * esz - 1)) == 0;     // element positions are multiples of 4
 #pragma unroll
@@ -1142,12 +1141,13 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
                     const float4 a = lds16f(from), b = lds16f(from + 128), c = lds16f(from + 256), d = lds16f(from + 384);
                     // what a code's place in its word multiplied
                     const bool upper = k4 && (q & 1);  // nibbles 4 .. 7 of the word
-                    const float m0 = mul * (upper ? code_unit<TY, WEIGHTED>(4) : code_unit<TY, WEIGHTED>(0));
-                    const float m1 = mul * (upper ? code_unit<TY, WEIGHTED>(5) : code_unit<TY, WEIGHTED>(1));
-                    const float m2 = mul * (upper ? code_unit<TY, WEIGHTED>(6) : code_unit<TY, WEIGHTED>(2));
-                    const float m3 = mul * (upper ? code_unit<TY, WEIGHTED>(7) : code_unit<TY, WEIGHTED>(3));
-                    const float v[4] = {fmaf((a.x + b.x) + (c.x + d.x), m0, bm), fmaf((a.y + b.y) + (c.y + d.y), m1, bm),
-                                        fmaf((a.z + b.z) + (c.z + d.z), m2, bm), fmaf((a.w + b.w) + (c.w + d.w), m3, bm)};
+                    const float m0 = unit_base * (upper ? code_unit<TY, WEIGHTED>(4) : code_unit<TY, WEIGHTED>(0));
+                    const float m1 = unit_base * (upper ? code_unit<TY, WEIGHTED>(5) : code_unit<TY, WEIGHTED>(1));
+                    const float m2 = unit_base * (upper ? code_unit<TY, WEIGHTED>(6) : code_unit<TY, WEIGHTED>(2));
+                    const float m3 = unit_base * (upper ? code_unit<TY, WEIGHTED>(7) : code_unit<TY, WEIGHTED>(3));
+                    // the mean is taken of the finished sum: codes and biases that cancel do so before anything is rounded
+                    const float v[4] = {fmaf((a.x + b.x) + (c.x + d.x), m0, bias_acc) * mm, fmaf((a.y + b.y) + (c.y + d.y), m1, bias_acc) * mm,
+                                        fmaf((a.z + b.z) + (c.z + d.z), m2, bias_acc) * mm, fmaf((a.w + b.w) + (c.w + d.w), m3, bias_acc) * mm};
                     constexpr int QPU = EPU / 4;       // quads of a unit
                     const int unit = u0 + xu + 8 * (q / QPU);
                     int e0 = EPU * unit - HS + 4 * (q % QPU);

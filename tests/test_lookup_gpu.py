@@ -481,3 +481,17 @@ def test_pieces_of_a_bag_are_added_without_their_cancelled_parts(weights_ty, D, 
     c = _one_table_of_rows(weights_ty, D, [(2.0 ** -10, 0.0), (32768.0 / big, -32768.0)], [small, np.full(D, big)],
                            [0] * 32 + [1] * 32, [0, 64], 1, np.ones(64, np.float32) if weighted else None)
     assert np.array_equal(gpu_lookup(c, O.SUM, O.FP32)[0], (small * 2.0 ** -5).astype(np.float32))
+
+
+@pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4])
+@pytest.mark.parametrize("D", [40, 128, 520])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_mean_of_rows_that_cancel_is_zero(weights_ty, D, weighted):
+    """Rows of code * scale - 32768 = 0: the codes' sum and the biases' sum are whole multiples of 2^15 and cancel exactly, so
+    their mean over 3, 5 or 7 rows is exactly zero; a bias that is divided (and rounded) by itself leaves a remainder.  9000
+    bags: a warp takes several in a row, whole ones and such that lane groups share."""
+    big = 64 if weights_ty == O.INT8 else 8
+    offsets = np.cumsum([0] + [3, 5, 7] * 3000)
+    c = _one_table_of_rows(weights_ty, D, [(32768.0 / big, -32768.0)], [np.full(D, big)], [0] * int(offsets[-1]), offsets, 9000,
+                           np.ones(int(offsets[-1]), np.float32) if weighted else None)
+    assert np.all(gpu_lookup(c, O.MEAN, O.FP32) == 0.0)
