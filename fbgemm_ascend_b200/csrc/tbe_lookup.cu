@@ -493,7 +493,7 @@ __host__ __device__ constexpr int floor_pow2(int x) { return x >= 8 ? 8 : x >= 4
 __host__ __device__ constexpr int min3(int a, int b, int c) { return a < b ? (a < c ? a : c) : (b < c ? b : c); }
 
 // A run of nb <= kMaxRunBags consecutive bags of ONE table whose rows are D = 16 * n <= 512 elements, 16-byte
-// aligned.  LPR lanes share a row, 16 elements per lane, so a warp has G = 32 / LPR lane groups.
+// aligned.  Lane l <= nb brings the offset of bag l relative to the run's first row, R0, as `rel`.  LPR lanes share a row, 16 elements per lane, so a warp has G = 32 / LPR lane groups.
 //
 // Work split.  The run's rows -- positions [R0, R1) of `indices` -- are cut into G equal ranges, one per
 // group, whatever the bag lengths are, so the groups finish together.  A group walks its range row by row
@@ -513,7 +513,7 @@ __host__ __device__ constexpr int min3(int a, int b, int c) { return a < b ? (a 
 // copied itself, so no barrier is involved.  A row that is not to be added (index -1, out of range, past the end
 // of the group's range) is zero-filled in the stage without being read.
 template <int TY, int LPR, int EPL, bool WEIGHTED>
-__device__ __forceinline__ void pool_run_stream(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
+__device__ __forceinline__ void pool_run_stream(const LookupParams& p, const TableMeta& m, int64_t R0, int rel, int nb, int64_t b0, int lane,
                                              uint32_t wsm)
 {
     static_assert(EPL == 16 || (EPL == 32 && (TY == TBE_B200_INT8 || TY == TBE_B200_INT4)), "32 elements per lane: INT8 / INT4 only");
@@ -547,22 +547,7 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
     const int isz = idx64 ? 8 : 4;
     const uint32_t sm_rel = wsm + kPartBytes;
 
-    // The run's nb + 1 offsets, one per lane, relative to the first one.
-    int64_t off = 0;
-    if (lane <= nb) {
-        const char* op = static_cast<const char*>(p.offsets) + (i0 + lane) * isz;
-        off = idx64 ? __ldg(reinterpret_cast<const int64_t*>(op)) : static_cast<int64_t>(__ldg(reinterpret_cast<const int32_t*>(op)));
-    }
-    int64_t R0 = __shfl_sync(kFull, off, 0);
-    int64_t R1 = __shfl_sync(kFull, off, nb);
-    if (R0 < 0 || R1 < R0 || R1 > p.num_indices || R1 - R0 > 0x7fffffffll) {
-        // Offsets that do not describe positions of `indices`: nothing is read through them; the run's bags are
-        // written as empty ones (zeros), so that the output is defined, and the condition is reported.
-        if (p.error_flag && lane == 0) atomicOr(p.error_flag, 8);
-        off = R0 = R1 = 0;
-    }
-    const int n = static_cast<int>(R1 - R0);
-    const int rel = static_cast<int>(min(max(off - R0, static_cast<int64_t>(0)), static_cast<int64_t>(n)));
+    const int n = __shfl_sync(kFull, rel, nb);
     __syncwarp();                                      // the previous run's reads of this memory are over
     if (lane <= nb) sts4(sm_rel + 4 * lane, rel);
     __syncwarp();
@@ -864,7 +849,7 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
 }
 
 template <int TY, bool WEIGHTED>
-__device__ __forceinline__ void pool_run_stream_by_width(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b,
+__device__ __forceinline__ void pool_run_stream_by_width(const LookupParams& p, const TableMeta& m, int64_t R0, int rel, int nb, int64_t b,
                                                          int lane, uint32_t wsm)
 {
     // INT8 / INT4 rows of 128 elements or more that divide into 32-element pieces: 32 elements per lane, so that twice
@@ -872,31 +857,31 @@ __device__ __forceinline__ void pool_run_stream_by_width(const LookupParams& p, 
     if constexpr (TY == TBE_B200_INT8 || TY == TBE_B200_INT4) {
         if (m.D >= 128 && (m.D & 31) == 0) {
             const int n32 = m.D / 32;
-            if (n32 <= 4) pool_run_stream<TY, 4, 32, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
-            else if (n32 <= 8) pool_run_stream<TY, 8, 32, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
-            else pool_run_stream<TY, 16, 32, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+            if (n32 <= 4) pool_run_stream<TY, 4, 32, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+            else if (n32 <= 8) pool_run_stream<TY, 8, 32, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+            else pool_run_stream<TY, 16, 32, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
             return;
         }
     }
     const int nunits = m.D / 16;
-    if (nunits <= 4) pool_run_stream<TY, 4, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
-    else if (nunits <= 8) pool_run_stream<TY, 8, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
-    else if (nunits <= 16) pool_run_stream<TY, 16, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
-    else pool_run_stream<TY, 32, 16, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+    if (nunits <= 4) pool_run_stream<TY, 4, 16, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+    else if (nunits <= 8) pool_run_stream<TY, 8, 16, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+    else if (nunits <= 16) pool_run_stream<TY, 16, 16, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+    else pool_run_stream<TY, 32, 16, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
 }
 
 template <bool WEIGHTED>
-__device__ __forceinline__ void pool_run_stream_by_type(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b,
+__device__ __forceinline__ void pool_run_stream_by_type(const LookupParams& p, const TableMeta& m, int64_t R0, int rel, int nb, int64_t b,
                                                         int lane, uint32_t wsm)
 {
     switch (m.ty) {
         case TBE_B200_INT8:
-            pool_run_stream_by_width<TBE_B200_INT8, WEIGHTED>(p, m, i0, nb, b, lane, wsm);
+            pool_run_stream_by_width<TBE_B200_INT8, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
             return;
-        case TBE_B200_INT4: pool_run_stream_by_width<TBE_B200_INT4, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
-        case TBE_B200_FP8: pool_run_stream_by_width<TBE_B200_FP8, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
-        case TBE_B200_FP16: pool_run_stream_by_width<TBE_B200_FP16, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
-        default: pool_run_stream_by_width<TBE_B200_FP32, WEIGHTED>(p, m, i0, nb, b, lane, wsm); return;
+        case TBE_B200_INT4: pool_run_stream_by_width<TBE_B200_INT4, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm); return;
+        case TBE_B200_FP8: pool_run_stream_by_width<TBE_B200_FP8, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm); return;
+        case TBE_B200_FP16: pool_run_stream_by_width<TBE_B200_FP16, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm); return;
+        default: pool_run_stream_by_width<TBE_B200_FP32, WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm); return;
     }
 }
 
@@ -927,7 +912,7 @@ __device__ __forceinline__ void cp_async4_if(bool on, uint32_t dst, const void* 
 constexpr int kIndexRing = 128;                        // rows whose numbers (and weights) are at hand: a power of two above what is in flight
 
 template <int TY, int CB, bool WEIGHTED>
-__device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane, uint32_t wsm)
+__device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMeta& m, int64_t R0, int rel, int nb, int64_t b0, int lane, uint32_t wsm)
 {
     static_assert(CB == 4 || CB == 8 || CB == 16 || (CB == 32 && TY != TBE_B200_INT4), "at most 32 elements per lane and pass");
     constexpr bool k8 = (TY == TBE_B200_INT8), k4 = (TY == TBE_B200_INT4), k16 = (TY == TBE_B200_FP16), kF8 = (TY == TBE_B200_FP8),
@@ -962,30 +947,9 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
     const int isz = idx64 ? 8 : 4;
     const uint32_t sm_rel = wsm, sm_idx = wsm + kRelBytes, sm_w = sm_idx + kIndexRing * 4, sm_x = sm_w + kIndexRing * 4, ring = sm_x + XCHG;
 
-    int64_t off = 0;
-    if (lane <= nb) {
-        const char* op = static_cast<const char*>(p.offsets) + (i0 + lane) * isz;
-        off = idx64 ? __ldg(reinterpret_cast<const int64_t*>(op)) : static_cast<int64_t>(__ldg(reinterpret_cast<const int32_t*>(op)));
-    }
-    int64_t R0 = __shfl_sync(kFull, off, 0);
-    int64_t R1 = __shfl_sync(kFull, off, nb);
-    if (R0 < 0 || R1 < R0 || R1 > p.num_indices || R1 - R0 > 0x7fffff00ll) {
-        // Offsets that do not describe positions of `indices`: nothing is read through them; the run's bags are
-        // written as empty ones (zeros), so that the output is defined, and the condition is reported.
-        if (p.error_flag && lane == 0) atomicOr(p.error_flag, 8);
-        off = R0 = R1 = 0;
-    }
-    const int n = static_cast<int>(R1 - R0);
-    int rel = static_cast<int>(min(max(off - R0, static_cast<int64_t>(0)), static_cast<int64_t>(n)));
-    if (lane > nb) rel = n;
-    // (offsets that run backwards inside the run count as the largest before them, so that the walk below only moves on)
-#pragma unroll
-    for (int d = 1; d < kWarp; d <<= 1) {
-        const int before = __shfl_up_sync(kFull, rel, d);
-        if (lane >= d) rel = max(rel, before);
-    }
+    const int n = __shfl_sync(kFull, rel, nb);
     __syncwarp();                                      // the previous run's reads of this memory are over
-    sts4(sm_rel + 4 * lane, rel);
+    if (lane <= nb) sts4(sm_rel + 4 * lane, rel);
     const int next_rel = __shfl_down_sync(kFull, rel, 1);
     const int total_steps = static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(lane < nb ? (next_rel - rel + 7) >> 3 : 0)));
     __syncwarp();
@@ -1211,7 +1175,7 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
 }
 
 template <int TY, bool WEIGHTED>
-__device__ __forceinline__ void pool_run_steps_by_width(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
+__device__ __forceinline__ void pool_run_steps_by_width(const LookupParams& p, const TableMeta& m, int64_t R0, int rel, int nb, int64_t b0, int lane,
                                                         uint32_t wsm)
 {
     // The narrowest unit with which eight lanes cover the row, so that narrow rows keep all of them busy.
@@ -1219,29 +1183,29 @@ __device__ __forceinline__ void pool_run_steps_by_width(const LookupParams& p, c
     const int bytes = TY == TBE_B200_FP32 ? 4 * m.D : TY == TBE_B200_FP16 ? 2 * m.D : TY == TBE_B200_INT4 ? m.D / 2 : m.D;
     auto covers = [&](int unit) { return bytes <= 8 * unit && (bytes % unit == 0 || bytes + kHead <= 8 * unit); };
     if constexpr (kHead != 0 || TY == TBE_B200_FP8) {
-        if (covers(4)) { pool_run_steps<TY, 4, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return; }
+        if (covers(4)) { pool_run_steps<TY, 4, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return; }
     }
     if constexpr (TY != TBE_B200_FP32) {
-        if (covers(8)) { pool_run_steps<TY, 8, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return; }
+        if (covers(8)) { pool_run_steps<TY, 8, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return; }
     }
     if constexpr (TY == TBE_B200_INT4) {
-        pool_run_steps<TY, 16, WEIGHTED>(p, m, i0, nb, b0, lane, wsm);
+        pool_run_steps<TY, 16, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm);
     } else {
-        if (covers(16)) pool_run_steps<TY, 16, WEIGHTED>(p, m, i0, nb, b0, lane, wsm);
-        else pool_run_steps<TY, 32, WEIGHTED>(p, m, i0, nb, b0, lane, wsm);
+        if (covers(16)) pool_run_steps<TY, 16, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm);
+        else pool_run_steps<TY, 32, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm);
     }
 }
 
 template <bool WEIGHTED>
-__device__ __forceinline__ void pool_run_steps_by_type(const LookupParams& p, const TableMeta& m, int64_t i0, int nb, int64_t b0, int lane,
+__device__ __forceinline__ void pool_run_steps_by_type(const LookupParams& p, const TableMeta& m, int64_t R0, int rel, int nb, int64_t b0, int lane,
                                                        uint32_t wsm)
 {
     switch (m.ty) {
-        case TBE_B200_INT8: pool_run_steps_by_width<TBE_B200_INT8, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
-        case TBE_B200_INT4: pool_run_steps_by_width<TBE_B200_INT4, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
-        case TBE_B200_FP8: pool_run_steps_by_width<TBE_B200_FP8, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
-        case TBE_B200_FP16: pool_run_steps_by_width<TBE_B200_FP16, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
-        default: pool_run_steps_by_width<TBE_B200_FP32, WEIGHTED>(p, m, i0, nb, b0, lane, wsm); return;
+        case TBE_B200_INT8: pool_run_steps_by_width<TBE_B200_INT8, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return;
+        case TBE_B200_INT4: pool_run_steps_by_width<TBE_B200_INT4, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return;
+        case TBE_B200_FP8: pool_run_steps_by_width<TBE_B200_FP8, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return;
+        case TBE_B200_FP16: pool_run_steps_by_width<TBE_B200_FP16, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return;
+        default: pool_run_steps_by_width<TBE_B200_FP32, WEIGHTED>(p, m, R0, rel, nb, b0, lane, wsm); return;
     }
 }
 
@@ -1338,15 +1302,26 @@ __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe
         }
         // the bags left in the span, in table t and at all
         const int nb = static_cast<int>(min(min(p.span - done, p.B - b), p.num_bags - i));
+        // The run's nb + 1 offsets, one per lane.
+        int64_t off = 0;
+        if (lane <= nb) {
+            const char* o = static_cast<const char*>(p.offsets) + (i + lane) * (p.idx64 ? 8 : 4);
+            off = p.idx64 ? __ldg(reinterpret_cast<const int64_t*>(o)) : static_cast<int64_t>(__ldg(reinterpret_cast<const int32_t*>(o)));
+        }
         const TableMeta m = load_meta(p, t);
-        const bool aligned = m.D > 0 && m.rows_aligned && (m.D & 3) == 0 && m.stride < (1ll << 32) &&
+        // A run with an offset that goes backwards or points outside `indices` (or one of 2^31 rows) is taken byte by byte, which
+        // looks at every bag: the bad ones are reported and left empty, the others come out as ever.
+        const int64_t R0 = __shfl_sync(kFull, off, 0), before = __shfl_up_sync(kFull, off, 1);
+        const bool sane = !__any_sync(kFull, lane <= nb && (off < before || off < 0 || off > p.num_indices || off - R0 > 0x7fffff00ll));
+        const int rel = static_cast<int>(off - R0);
+        const bool aligned = sane && m.D > 0 && m.rows_aligned && (m.D & 3) == 0 && m.stride < (1ll << 32) &&
                              (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32 ||
                               (m.ty == TBE_B200_FP8 && p.fp8_shift <= 23));
         // Widths that give every lane of a row the same 16 elements go through the streams, which issue a third fewer instructions
         // there (64 INT8 tables of 128: 3.63 ms against 6.0 in steps; INT4 of 64/128/256: 1.23 against 1.91 ms); all others in
         // steps (16 tables of 20 to 1024 elements of four types: 174 us; 338 us one bag at a time or byte by byte).
-        if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
-        else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, i, nb, b, lane, wsm);
+        if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+        else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
         else if (m.D > 0 && p.idx64) pool_run_bytewise<int64_t>(p, m, i, nb, b, lane);
         else if (m.D > 0) pool_run_bytewise<int32_t>(p, m, i, nb, b, lane);
         done += nb;

@@ -495,3 +495,43 @@ def test_mean_of_rows_that_cancel_is_zero(weights_ty, D, weighted):
     c = _one_table_of_rows(weights_ty, D, [(32768.0 / big, -32768.0)], [np.full(D, big)], [0] * int(offsets[-1]), offsets, 9000,
                            np.ones(int(offsets[-1]), np.float32) if weighted else None)
     assert np.all(gpu_lookup(c, O.MEAN, O.FP32) == 0.0)
+
+
+@pytest.mark.parametrize("weights_ty", [O.INT8, O.FP16])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("dims", [[20, 128, 528], [64, 128, 256], [20, 36, 1]])
+def test_bad_offsets_inside_a_run_are_reported_bag_by_bag(weights_ty, weighted, dims):
+    """Offsets that go backwards, past the end of `indices` or below zero between good ones (8000 bags per table: a warp takes
+    eleven in a row): bit 8, the bags they bound come out as zeros, and every other bag as if nothing had happened."""
+    import torch
+    from fbgemm_ascend_b200 import cabi
+
+    rng = np.random.default_rng(seed_of("bad offsets", weights_ty, weighted, dims))
+    T, B = 3, 8000
+    c = make_case(rng, [weights_ty] * T, dims, [100] * T, B, rng.integers(0, 5, T * B), np.int64, weighted)
+    n = c.indices.size
+    for t in range(T):
+        for b, value in ((4, 10 ** 9), (1003, -7), (4007, None), (6000, n + 1)):
+            i = t * B + b
+            c.offsets[i] = c.offsets[i - 1] - 3 if value is None else value
+    start, end = c.offsets[:-1], c.offsets[1:]
+    sane = (start >= 0) & (end >= start) & (end <= n)
+    assert int((~sane).sum()) == 7 * T
+    # the good bags, one after the other (the one behind a backward step has its neighbour's last three rows as well)
+    pieces = [slice(int(s), int(e)) if ok else slice(0, 0) for s, e, ok in zip(start, end, sane)]
+    idx = np.concatenate([c.indices[p] for p in pieces])
+    offsets = np.concatenate([[0], np.cumsum([p.stop - p.start for p in pieces])]).astype(np.int64)
+    good = Case(c.dev_weights, c.weights_offsets, c.weights_tys, c.D_offsets, idx, offsets,
+                None if c.weights is None else np.concatenate([c.weights[p] for p in pieces]), c.tys, c.dims, c.rows, B)
+    d = torch.device("cuda")
+    t_ = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(d)
+    flag = torch.zeros(1, dtype=torch.int32, device=d)
+    out = torch.full((B, c.total_D), 7.0, dtype=torch.float32, device=d)
+    cabi.lookup(t_(c.dev_weights), t_(c.weights_offsets), t_(c.weights_tys), t_(c.D_offsets), c.total_D, max(dims), t_(c.indices),
+                t_(c.offsets), O.SUM, out, indice_weights=None if c.weights is None else t_(c.weights), error_flag=flag)
+    assert int(flag.item()) == 8
+    got, want = out.cpu().numpy(), _pool_64(good, O.SUM)
+    assert np.all(np.abs(got - want[0]) <= want[1] * (2.0 ** -22 + 2.0 ** -23 * np.diff(offsets).reshape(T, B).T.repeat(dims, axis=1)) + 1e-38)
+    for t in range(T):
+        bad = ~sane[t * B:(t + 1) * B]
+        assert np.all(got[bad][:, c.D_offsets[t]:c.D_offsets[t + 1]] == 0.0)
