@@ -535,3 +535,13 @@ def test_bad_offsets_inside_a_run_are_reported_bag_by_bag(weights_ty, weighted, 
     for t in range(T):
         bad = ~sane[t * B:(t + 1) * B]
         assert np.all(got[bad][:, c.D_offsets[t]:c.D_offsets[t + 1]] == 0.0)
+
+
+@pytest.mark.parametrize("weights_ty", [O.INT8, O.INT4, O.FP16, O.FP8, O.FP32])
+@pytest.mark.parametrize("dims", [[16, 20], [16, 18], [16, 17], [128, 132], [136, 140]])
+@pytest.mark.parametrize("out_ty", [O.FP32, O.FP16, O.BF16])
+def test_sequence_rows_that_are_not_whole_pieces(weights_ty, dims, out_ty):
+    """Output rows that start on 8, 4 or 2 bytes (widths of an even table set by an odd one beside it)."""
+    rng = np.random.default_rng(seed_of("sequence rows", weights_ty, dims))
+    c = make_case(rng, [weights_ty] * 2, dims, [70] * 2, 3, np.array([40, 64, 3, 9, 0, 70]), np.int64, False, prune_frac=0.05)
+    run(c, O.NONE, out_ty, f"sequence dims={dims}")
