@@ -7,7 +7,7 @@
 // its columns measured slower than the packed FMAs: the instruction runs at one per 64 cycles and SM quarter here.
 //
 // Pooled kernel (SUM / MEAN), in three tiers chosen per table:
-//   * aligned rows of INT8 / INT4 / FP8 / FP16 / FP32 with D a multiple of 16 up to 512 (pool_run_stream): LPR lanes
+//   * aligned rows of INT8 / INT4 / FP8 / FP16 / FP32 with D a multiple of 16 up to 512 (FP32: from 80) (pool_run_stream): LPR lanes
 //     share a row, 16 fp32 accumulators per lane, so a warp has 32/LPR lane groups.  The rows of a warp's bags are
 //     cut into equal ranges, one per group, and every group streams its range through a small ring in shared
 //     memory: asynchronous 16-byte copies through L1 (which holds the hot head of a Zipf-distributed table), several
@@ -1328,10 +1328,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe
         const bool aligned = sane && m.D > 0 && m.rows_aligned && (m.D & 3) == 0 && m.stride < (1ll << 32) &&
                              (m.ty == TBE_B200_INT8 || m.ty == TBE_B200_INT4 || m.ty == TBE_B200_FP16 || m.ty == TBE_B200_FP32 ||
                               (m.ty == TBE_B200_FP8 && p.fp8_shift <= 23));
-        // Widths that give every lane of a row the same 16 elements go through the streams, which issue a third fewer instructions
-        // there (64 INT8 tables of 128: 3.63 ms against 6.0 in steps; INT4 of 64/128/256: 1.23 against 1.91 ms); all others in
-        // steps (16 tables of 20 to 1024 elements of four types: 174 us; 338 us one bag at a time or byte by byte).
-        if (aligned && (m.D & 15) == 0 && m.D <= 512) pool_run_stream_by_type<WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
+        // Aligned widths of 16 n <= 512 elements go through the streams, fp32 rows of up to 64 elements and all other widths in
+        // steps.  24 tables of 200 K rows, batch 4096, bags of 32, fp16 result, streams against steps in us: INT8 of 16, 48, 128,
+        // 144, 512 elements 72, 76, 127, 187, 322 against 126, 134, 154, 197, 494; FP16 75, 97, 134, 200, 490 against 106, 121, 155,
+        // 310, 585; FP8 97, 88, 132, 226, 412 against 119, 128, 152, 230, 446; INT4 85, 79, 108, 194, 267 against 143, 134, 150, 185, 393
+        // (144 and 208 INT4 elements alone would be 4 % faster in steps); FP32 of 16, 32, 48, 64, 80, 128 elements 120, 124, 140, 138,
+        // 210, 253 against 107, 109, 137, 134, 267, 263.
+        const bool stream = aligned && (m.D & 15) == 0 && m.D <= 512 && !(m.ty == TBE_B200_FP32 && m.D <= 64);
+        if (stream) pool_run_stream_by_type<WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
         else if (aligned) pool_run_steps_by_type<WEIGHTED>(p, m, R0, rel, nb, b, lane, wsm);
         else if (m.D > 0 && p.idx64) pool_run_bytewise<int64_t>(p, m, i, nb, b, lane);
         else if (m.D > 0) pool_run_bytewise<int32_t>(p, m, i, nb, b, lane);

@@ -351,8 +351,9 @@ def _pool_64(c, pooling):
             head = rows[:, :4].copy().view(np.float16).astype(np.float64)
             scale, bias = head[:, :1], head[:, 1:]
             codes = rows[:, 4:4 + D] if ty == O.INT8 else np.stack([rows[:, 4:4 + D // 2] & 15, rows[:, 4:4 + D // 2] >> 4], 2).reshape(E, D)
-        elif ty == O.FP16:
-            codes = rows[:, :2 * D].copy().view(np.float16)
+        elif ty in (O.FP16, O.FP32):
+            dt = np.dtype(np.float16 if ty == O.FP16 else np.float32)
+            codes = rows[:, :dt.itemsize * D].copy().view(dt)
         else:
             b = rows[:, :D].astype(np.int64)
             e, m = (b >> 3) & 15, (b & 7) / 8.0
@@ -373,7 +374,7 @@ def _pool_64(c, pooling):
     (O.INT8, [4, 28, 32, 36, 60, 64]), (O.INT8, [68, 124, 128, 132]), (O.INT8, [252, 256, 260, 516]),
     (O.INT4, [8, 56, 64, 72, 120, 128]), (O.INT4, [136, 248, 256, 264, 520]),
     (O.FP8, [4, 32, 36, 64, 68]), (O.FP8, [128, 132, 256, 260]),
-    (O.FP16, [4, 12, 16, 32, 36]), (O.FP16, [64, 68, 128, 132, 260])])
+    (O.FP16, [4, 12, 16, 32, 36]), (O.FP16, [64, 68, 128, 132, 260]), (O.FP32, [4, 16, 32, 36, 48, 64]), (O.FP32, [68, 80, 128, 132, 260])])
 @pytest.mark.parametrize("weighted", [False, True])
 @pytest.mark.parametrize("out_ty", [O.FP32, O.FP16, O.BF16])
 def test_row_widths_at_the_edges_of_the_units(weights_ty, dims, weighted, out_ty):
