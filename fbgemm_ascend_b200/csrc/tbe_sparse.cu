@@ -418,9 +418,12 @@ __global__ void __launch_bounds__(kBigThreads, kBigBlocksPerSM) big_tile_scan_ke
 constexpr int kMaxPartials = 32;             // blocks that add up one table's lengths
 constexpr int kOffsetThreads = 256;
 constexpr int kSmallThreads = 1024;
-// The one-block form takes up to this many tables, lengths per table and lengths in all: a warp then reads at most 16
-// lines of a table, and four tables one after the other, which is what the launches it saves cost.
-constexpr int64_t kSmallTables = 128, kSmallBatch = 512, kSmallLengths = 16384;
+// The one-block form takes up to this many tables, lengths per table and lengths in all.  On the device the two launches are
+// never slower; one launch less is what a caller saves whose kernels are shorter than their launches.  Calls one after the
+// other / in a graph, us, one block against two launches, values of int64 in bags of 30: 26 tables x 64 12.9 / 9.6 against 15.8 / 9.4,
+// 26 x 256 13.8 / 10.7 against 15.0 / 9.6, 64 x 64 16.5 / 11.9 against 16.5 / 10.5, 64 x 128 16.8 / 13.1 against 16.7 / 10.3; beyond
+// that the block is too slow: 64 x 256 17.8 / 13.9 against 16.4 / 10.9, 128 x 128 20.8 / 17.0 against 16.6 / 11.4.
+constexpr int64_t kSmallTables = 64, kSmallBatch = 512, kSmallLengths = 8192;
 inline bool small_request(int64_t T_in, int64_t T_out, int64_t B)
 {
     return T_in <= kSmallTables && T_out <= kSmallTables && B <= kSmallBatch && T_in * B <= kSmallLengths && T_out * B <= kSmallLengths;

@@ -263,7 +263,8 @@ def test_permute_2d_sparse_data_shapes(shape, wcols):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("t_in,t_out,b", [(1, 1, 512), (1, 3, 513), (32, 32, 512), (33, 20, 512), (128, 128, 128), (129, 128, 4), (128, 129, 4),
+@pytest.mark.parametrize("t_in,t_out,b", [(1, 1, 512), (1, 3, 513), (32, 32, 512), (33, 20, 512), (16, 16, 512), (17, 16, 512), (64, 64, 128), (64, 64, 129), (65, 64, 4),
+                                          (64, 65, 4), (128, 128, 128), (129, 128, 4), (128, 129, 4),
                                           (3, 2, 2048), (3, 2, 2049), (2, 5, 70000), (300, 257, 60)])
 @pytest.mark.parametrize("vname", ["int64", "int32", "float16"])
 def test_permute_2d_at_the_edges_of_its_forms(t_in, t_out, b, vname):
