@@ -81,35 +81,39 @@ __host__ __device__ inline int64_t row_bytes_of(int ty, int D, int align)
 
 // ---- output ----------------------------------------------------------------
 
-// Converts and stores N (1, 2 or 4) consecutive finished elements.  `p` points at
-// the first of them in the output, already offset; `vec` says the address is
-// aligned for one N-wide store.
-template <int N>
-__device__ __forceinline__ void store_out(void* seg, int e0, const float* v, int out_ty, bool vec)
+// Two finished elements as 16-bit ones.
+__device__ __forceinline__ uint32_t pack_out(float a, float b, int out_ty)
+{
+    if (out_ty == TBE_B200_FP16) {
+        const __half2 x = __floats2half2_rn(a, b);
+        return *reinterpret_cast<const uint32_t*>(&x);
+    }
+    const __nv_bfloat162 x = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&x);
+}
+
+// Converts and stores four consecutive finished elements, from element e0 of `seg` on; `vec` says that the address is
+// aligned for one store.
+__device__ __forceinline__ void store_out4(void* seg, int e0, const float* v, int out_ty, bool vec)
 {
     if (out_ty == TBE_B200_FP32) {
         float* p = static_cast<float*>(seg) + e0;
-        if (N == 4 && vec) {
-            st_stream16(p, make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]),
-                                      __float_as_uint(v[3])));
-        } else if (N == 2 && vec) {
-            st_stream8(p, make_uint2(__float_as_uint(v[0]), __float_as_uint(v[1])));
+        if (vec) {
+            st_stream16(p, make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])));
         } else {
 #pragma unroll
-            for (int j = 0; j < N; ++j) p[j] = v[j];
+            for (int j = 0; j < 4; ++j) p[j] = v[j];
         }
     } else {
-        uint32_t h[N];
+        uint32_t h[4];
 #pragma unroll
-        for (int j = 0; j < N; ++j) h[j] = (out_ty == TBE_B200_FP16) ? f32_to_f16_bits(v[j]) : f32_to_bf16_bits(v[j]);
+        for (int j = 0; j < 4; ++j) h[j] = (out_ty == TBE_B200_FP16) ? f32_to_f16_bits(v[j]) : f32_to_bf16_bits(v[j]);
         unsigned short* p = static_cast<unsigned short*>(seg) + e0;
-        if (N == 4 && vec) {
+        if (vec) {
             st_stream8(p, make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16)));
-        } else if (N == 2 && vec) {
-            st_stream4(p, h[0] | (h[1] << 16));
         } else {
 #pragma unroll
-            for (int j = 0; j < N; ++j) p[j] = static_cast<unsigned short>(h[j]);
+            for (int j = 0; j < 4; ++j) p[j] = static_cast<unsigned short>(h[j]);
         }
     }
 }
@@ -171,13 +175,11 @@ __device__ __forceinline__ uint32_t lds4(uint32_t a)
 
 // ---- dequantisation arithmetic ------------------------------------------------
 //
-// Integer -> float conversion instructions run at 16 lanes per clock per SM on sm_100a, which
-// would cap a 128-element INT8 row at 8 cycles.  Codes are therefore turned into exact fp16 values
-// with one byte permute (or mask) and one half2 subtract per pair -- 0x6400 | q is the half 1024 + q
-// -- and accumulated with the sm_100 mixed-precision FMA (fp16 * fp16 + fp32 -> fp32): the row scale
-// is stored as fp16, so code * scale is formed exactly and added to the fp32 accumulator with a
-// single rounding, as an fp32 FMA would.  With per-sample weights the scale is no longer an fp16
-// value; the codes are then widened to fp32 and an fp32 FMA with w * scale is used.
+// Integer -> float conversion instructions run at 16 lanes per clock per SM on sm_100a, which would cap a 128-element INT8
+// row at 8 cycles, so neither mode uses them.  Pooled sums take codes where they lie (see kCodeScale).  Sequence mode
+// turns codes into exact fp16 values with one byte permute (or mask) and one half2 subtract per pair -- 0x6400 | q is the
+// half 1024 + q -- and adds them to the bias with the sm_100 mixed-precision FMA (fp16 * fp16 + fp32 -> fp32): the
+// row scale is stored as fp16, so code * scale + bias is rounded once, as by an fp32 FMA.
 
 // Two exact fp16 values (as a half2 bit pattern) from two codes already or'ed into the mantissas of
 // the half2 `magic` (0x6400: 1024, 0x5400: 64 with the code in mantissa bits 4..7).
@@ -187,19 +189,12 @@ __device__ __forceinline__ uint32_t codes_to_half2(uint32_t packed, uint32_t mag
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// acc[0..1] += pair (half2 bits) * scale: mixed FMA with the fp16 scale, or fp32 FMA with `ws`.
-template <bool WEIGHTED>
-__device__ __forceinline__ void add_pair_t(float& a0, float& a1, uint32_t pair, unsigned short scale_h, float ws)
+// a0, a1 += pair (half2 bits) * scale (fp16 bits), a mixed FMA each.
+__device__ __forceinline__ void add_pair(float& a0, float& a1, uint32_t pair, unsigned short scale_h)
 {
-    if constexpr (!WEIGHTED) {
-        asm("{ .reg .b16 l, h; mov.b32 {l, h}, %2; fma.rn.f32.f16 %0, l, %3, %0; fma.rn.f32.f16 %1, h, %3, %1; }"
-            : "+f"(a0), "+f"(a1)
-            : "r"(pair), "h"(scale_h));
-    } else {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&pair));
-        a0 = fmaf(f.x, ws, a0);
-        a1 = fmaf(f.y, ws, a1);
-    }
+    asm("{ .reg .b16 l, h; mov.b32 {l, h}, %2; fma.rn.f32.f16 %0, l, %3, %0; fma.rn.f32.f16 %1, h, %3, %1; }"
+        : "+f"(a0), "+f"(a1)
+        : "r"(pair), "h"(scale_h));
 }
 
 // Description of the table a bag belongs to; reloaded only when the warp moves on to another table.
@@ -394,8 +389,8 @@ __device__ __forceinline__ float2 fma2_value(float a0, float a1, float b0, float
 // the codes are made ordinary numbers first: a nibble that lies at bit k becomes 2^(23 - k) + q in the masking instruction, less
 // 2^(23 - k) in half a packed addition (a byte 2^23 + q by a byte permute); the sums are then those of the codes themselves, and
 // overflow where fp32 does.
-// A step of eight 128-byte rows takes 162 instructions instead of 177 with a byte permute and a mixed FMA per code: 64 INT8
-// tables of 128, batch 65536: 3.83 -> 3.78 ms; INT4 of 64/128/256: 1.52 -> 1.41 ms.
+// Against a byte permute and a mixed FMA per code, and with the row loop inlined (see the kernel): 64 INT8 tables of 128, batch
+// 65536: 4.05 -> 3.38 ms; INT4 of 64/128/256, batch 16384: 1.73 -> 1.24 ms.
 constexpr float kCodeScale = 0x1p111f;
 template <int TY, bool WEIGHTED>
 __device__ constexpr float code_unit(int slot)
@@ -453,8 +448,8 @@ __device__ __forceinline__ void accum_codes(const uint32_t (&words)[NW], float s
 // fp8_mult, a power of two.  Unweighted sums get it at the bag's end (placed values are whole multiples of 2^-132 at least,
 // so nothing is lost below the normal range).  A weight may have any magnitude: there the values get it before they
 // meet the weight `w`.
-// 16 tables of 128 FP8, batch 8192: 212 -> 165 us against placing, scaling and signing every byte by itself (D = 256 with
-// weights: 426 -> 316).
+// Against placing, scaling and signing every byte by itself, 24 tables, 3.1 M rows: 128 elements 200 -> 132 us, 256 elements with
+// weights 364 -> 251 us.
 template <bool WEIGHTED, int NW>
 __device__ __forceinline__ void accum_fp8(const uint32_t (&words)[NW], uint32_t fp8_shift, float fp8_mult, float w, float* acc)
 {
@@ -635,15 +630,7 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
             if (vec && esz == 2) {
                 uint32_t h[EPL / 2];
 #pragma unroll
-                for (int q = 0; q < EPL / 2; ++q) {
-                    if (p.out_ty == TBE_B200_FP16) {
-                        const __half2 hh = __floats2half2_rn(acc[2 * q], acc[2 * q + 1]);
-                        h[q] = *reinterpret_cast<const uint32_t*>(&hh);
-                    } else {
-                        const __nv_bfloat162 bb = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
-                        h[q] = *reinterpret_cast<const uint32_t*>(&bb);
-                    }
-                }
+                for (int q = 0; q < EPL / 2; ++q) h[q] = pack_out(acc[2 * q], acc[2 * q + 1], p.out_ty);
                 const int from = (k + 1 == nunits) ? 0 : k + 1;
 #pragma unroll
                 for (int c = 0; c < NCH; ++c) {
@@ -663,7 +650,7 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
         }
         if (!stored && act) {
 #pragma unroll
-            for (int q = 0; q < EPL / 4; ++q) store_out<4>(seg, elem_of(4 * q), &acc[4 * q], p.out_ty, vec);
+            for (int q = 0; q < EPL / 4; ++q) store_out4(seg, elem_of(4 * q), &acc[4 * q], p.out_ty, vec);
         }
     };
     // Hands this group's settled piece of a bag that started in an earlier group's range to that bag's owner.
@@ -778,7 +765,7 @@ __device__ __forceinline__ void pool_run_stream(const LookupParams& p, const Tab
         } else if constexpr (TY == TBE_B200_FP16 && !WEIGHTED) {
             // value * 1.0 + acc in one mixed FMA
 #pragma unroll
-            for (int i8 = 0; i8 < 8; ++i8) add_pair_t<false>(acc[2 * i8], acc[2 * i8 + 1], r[i8], 0x3c00u, w);
+            for (int i8 = 0; i8 < 8; ++i8) add_pair(acc[2 * i8], acc[2 * i8 + 1], r[i8], 0x3c00u);
         } else if constexpr (TY == TBE_B200_FP16) {
 #pragma unroll
             for (int i8 = 0; i8 < 8; ++i8) {
@@ -1127,7 +1114,7 @@ __device__ __noinline__ void pool_run_steps(const LookupParams& p, const TableMe
                     const int unit = u0 + xu + 8 * (q / QPU);
                     int e0 = EPU * unit - HS + 4 * (q % QPU);
                     if (kHdr && unit == 0 && q % QPU < HS / 4) e0 = wrap ? D - HS + 4 * q : -1;
-                    if (unit < units && e0 >= 0 && e0 < D) store_out<4>(seg, e0, v, p.out_ty, vec);
+                    if (unit < units && e0 >= 0 && e0 < D) store_out4(seg, e0, v, p.out_ty, vec);
                 }
             }
 #pragma unroll
@@ -1264,10 +1251,9 @@ constexpr int kStreamBlocksPerSM = TBE_STREAM_BLOCKS_PER_SM;
 // warp walks `offsets`, `indices` and the per-sample weights front to back.  A span is processed as runs
 // of consecutive bags of one table: the table's description is read once per run and the run is handed
 // to the code specialised for its row shape.  pool_run_stream is inlined here (in a function of its own every memory
-// instruction has its descriptor moved into uniform registers again and the arguments are read through a pointer: 206
-// instead of 177 instructions per step of eight 128-byte rows); what a run does not need is not kept across it but
-// computed anew behind it, which leaves the row loop without spills (with them the loop is slower than the function was).
-// 64 INT8 tables of 128, batch 65536: 4.05 -> 3.83 ms; INT4 of 64/128/256: 1.72 -> 1.52 ms.
+// instruction has its descriptor moved into uniform registers again and the arguments are read through a pointer); what a run
+// does not need is not kept across it but computed anew behind it, which leaves the row loop without spills (with them the
+// loop is slower than the function was).  What this and the arithmetic at kCodeScale gave together stands there.
 template <bool WEIGHTED>
 __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, kStreamBlocksPerSM) tbe_pooled_kernel(const __grid_constant__ LookupParams p)
 {
@@ -1381,17 +1367,6 @@ __device__ __noinline__ void nobag_position_bytewise(const LookupParams& p, cons
     for (int e = m.D + lane; e < max_D; e += kWarp) store_scalar(seg, e, 0.0f, p.out_ty);
 }
 
-// Two finished elements as 16-bit ones.
-__device__ __forceinline__ uint32_t pack_out(float a, float b, int out_ty)
-{
-    if (out_ty == TBE_B200_FP16) {
-        const __half2 x = __floats2half2_rn(a, b);
-        return *reinterpret_cast<const uint32_t*>(&x);
-    }
-    const __nv_bfloat162 x = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&x);
-}
-
 // Stores 16 bytes with the widest stores that their address takes.  (Output rows need not start on 16 bytes: 128 elements
 // beside a table of 130 or 132, say.)
 __device__ __forceinline__ void store_piece(char* dst, const uint32_t (&h)[4])
@@ -1499,8 +1474,8 @@ __device__ __forceinline__ void nobag_pieces(const LookupParams& p, const TableM
                         const uint32_t c = raw[u][w];
                         const uint32_t even = codes_to_half2((c & 0x00FF00FFu) | 0x64006400u, 0x64006400u);
                         const uint32_t odd = codes_to_half2(__byte_perm(c, 0x64646464u, 0x4341), 0x64006400u);
-                        add_pair_t<false>(v[4 * w + 0], v[4 * w + 2], even, scale_h, 0.0f);
-                        add_pair_t<false>(v[4 * w + 1], v[4 * w + 3], odd, scale_h, 0.0f);
+                        add_pair(v[4 * w + 0], v[4 * w + 2], even, scale_h);
+                        add_pair(v[4 * w + 1], v[4 * w + 3], odd, scale_h);
                     }
                 } else {
                     // nibble pairs (j, j + EP / 2) are brought 16 bits apart
@@ -1508,13 +1483,13 @@ __device__ __forceinline__ void nobag_pieces(const LookupParams& p, const TableM
                     const uint32_t y = c >> 8;
                     const uint32_t p0 = codes_to_half2((c & 0x000F000Fu) | 0x64006400u, 0x64006400u);
                     const uint32_t p1 = codes_to_half2((c & 0x00F000F0u) | 0x54005400u, 0x54005400u);
-                    add_pair_t<false>(v[0], v[EP / 2], p0, scale_h, 0.0f);
-                    add_pair_t<false>(v[1], v[EP / 2 + 1], p1, scale_h, 0.0f);
+                    add_pair(v[0], v[EP / 2], p0, scale_h);
+                    add_pair(v[1], v[EP / 2 + 1], p1, scale_h);
                     if constexpr (EP == 8) {
                         const uint32_t p2 = codes_to_half2((y & 0x000F000Fu) | 0x64006400u, 0x64006400u);
                         const uint32_t p3 = codes_to_half2((y & 0x00F000F0u) | 0x54005400u, 0x54005400u);
-                        add_pair_t<false>(v[2], v[6], p2, scale_h, 0.0f);
-                        add_pair_t<false>(v[3], v[7], p3, scale_h, 0.0f);
+                        add_pair(v[2], v[6], p2, scale_h);
+                        add_pair(v[3], v[7], p3, scale_h);
                     }
                 }
             } else if constexpr (TY == TBE_B200_FP8) {
@@ -1539,7 +1514,7 @@ __device__ __forceinline__ void nobag_pieces(const LookupParams& p, const TableM
                 store_piece(dst, h);
             } else if (vec && (k_u[u] + 1) * EP <= width) {
                 if constexpr (EP == 4) {
-                    store_out<4>(dst, 0, v, TBE_B200_FP32, true);
+                    store_out4(dst, 0, v, TBE_B200_FP32, true);
                 } else {
                     uint32_t h[4];
 #pragma unroll

@@ -4,7 +4,7 @@ A lookup over tens of gigabytes of table rows cannot be repeated on the CPU in f
 (table, bag) pairs is checked instead: the rows those bags reference are copied to the host, the
 indices are renumbered onto that compact set of rows, the CPU oracle pools the compact case, and the
 result is compared with the corresponding slices of the GPU output.  The sample always contains the
-longest bags of the batch, because the error of fp32 accumulation (and of the folded INT8 form) grows
+longest bags of the batch, because the error of fp32 accumulation grows
 with the bag length.  The tolerances are the ones the reference's test uses
 (test_int_nbit_split_embedding_codegen_lookup_function.py:358-363).
 

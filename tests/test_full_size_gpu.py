@@ -74,7 +74,7 @@ def test_config2_full_against_oracle():
         err = np.abs(got - want)
         assert np.all(err <= 1e-3 + 1e-3 * np.abs(want)), f"c2 batch {seed}: max err {err.max():.3e}"
         lens = np.diff(b.offsets.cpu().numpy())
-        assert lens.max() >= 45        # long bags of the folded INT8 -> fp16 path are in the batch
+        assert lens.max() >= 45        # long bags are in the batch
     del tables
     torch.cuda.empty_cache()
 
@@ -97,13 +97,13 @@ def test_large_config_sampled_against_oracle(name):
         assert r["ok"], f"{name} {idx.dtype}: {r}"
         assert r["bags"] >= 4096
         if name == "c4":
-            assert r["max_len"] >= 60, r     # the tail of Poisson(32): the long bags of the folded path
+            assert r["max_len"] >= 60, r     # the tail of Poisson(32)
         if name == "c5":
             assert r["max_len"] == 200, r
         del out
     if name == "c4":
         # Poisson(32) hardly ever gives a bag of more than 70 rows; the configuration allows up to 128.  The same tables
-        # with bags of 100 to 128 rows (a smaller batch) put the folded INT8 -> fp16 accumulation at its longest.
+        # with bags of 100 to 128 rows (a smaller batch) put the INT8 -> fp16 accumulation at its longest.
         ws.length_dist = "uniform:100:128"
         ws.B = 4096
         bl = W.make_batch(ws, tables.device, batch_seed=7)
