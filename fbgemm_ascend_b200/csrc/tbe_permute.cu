@@ -7,12 +7,14 @@
 // One thread owns one VB-byte vector of output columns (16 bytes, or 8, 4 or 2 where the rows are not 16-byte
 // aligned) for kRows consecutive rows: it finds the output feature holding its first column once (binary search
 // of inv_offset_dim_list), then issues kRows independent loads and stores.  A vector whose source is not
-// VB-byte aligned, or that straddles features, is put together from two or four smaller pieces, each whole
-// in one feature, whose addresses are also found once; only a vector that does not divide into such pieces
-// (features of an odd number of 16-bit elements) is copied element by element.  So any dims are accepted and
+// VB-byte aligned, or that straddles features, is put together from two, four or eight smaller pieces, each whole
+// in one feature, whose addresses are also found once; only a vector that reaches past the last column or into an
+// invalid feature is copied element by element.  So any dims are accepted and
 // the host never has to read the lists (the reference syncs on them at
 // permute_pooled_embs.cpp:82-92).  Zero-width features are skipped.  Forward and backward of [8192, 10.4 K] fp16 with
 // features of 20, 36 and 100 elements: 475 us element by element, 149 us in pieces (a copy of the same bytes: 104 us).
+// Forward of [8192, 1536] fp16 with features of 3 elements: 56 us element by element, 59.5 us where 16-, 8- and 4-byte
+// pieces were tried before that, 29 us with 2-byte pieces; [4096, 8256] with features of 129: 112, 102 and 64 us.
 #include "tbe_common.cuh"
 
 namespace tbe {
@@ -131,6 +133,9 @@ __global__ void __launch_bounds__(kThreads) permute_pooled_embs_kernel(const Per
     }
     if constexpr (VB >= 8) {
         if (copy_pieces<VB, 4>(p, i, c0, row0, nrows)) return;
+    }
+    if constexpr (VB >= 4) {
+        if (p.esz == 2 && copy_pieces<VB, 2>(p, i, c0, row0, nrows)) return;
     }
 
     // Element-wise: walk the (possibly several) features this vector touches.
